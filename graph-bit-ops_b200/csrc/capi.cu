@@ -84,6 +84,28 @@ cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t s) {
   return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
+namespace {
+struct Pinned {
+  void* p = nullptr;
+  ~Pinned() {
+    if (p) cudaFreeHost(p);
+  }
+};
+}  // namespace
+
+cudaError_t read_back(void* dst, const void* d_src, size_t bytes, cudaStream_t s) {
+  static thread_local Pinned buf;
+  if (!buf.p && cudaHostAlloc(&buf.p, kReadBackBytes, cudaHostAllocPortable) != cudaSuccess) {
+    buf.p = nullptr;
+    (void)cudaGetLastError();
+  }
+  void* to = buf.p && bytes <= kReadBackBytes ? buf.p : dst;
+  cudaError_t e = cudaMemcpyAsync(to, d_src, bytes, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && to != dst) memcpy(dst, to, bytes);
+  return e;
+}
+
 int num_sms() {
   static thread_local int cached = 0;
   if (cached == 0) {

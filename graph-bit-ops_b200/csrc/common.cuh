@@ -94,6 +94,13 @@ inline cudaError_t pool_malloc_async(T** p, size_t bytes, cudaStream_t s) {
   return pool_malloc_async(reinterpret_cast<void**>(p), bytes, s);
 }
 
+// Copy a small device record (at most kReadBackBytes) to the host and wait
+// for the stream: through page-locked memory of the calling thread, which
+// the copy engine writes directly (a copy into pageable memory is staged by
+// the driver).
+constexpr size_t kReadBackBytes = 4096;
+cudaError_t read_back(void* dst, const void* d_src, size_t bytes, cudaStream_t s);
+
 // Host-side fault injection (gbo_debug_inject): true when this host CSR
 // allocation is the one armed to fail; the replay cap of the iteration
 // loops (0: none); whether server workers hold admission.

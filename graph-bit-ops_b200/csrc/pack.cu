@@ -11,6 +11,9 @@
 // entries in block column m into its tile row word, and the group emits one
 // tile.  A count pass sizes each block row; a scan gives bsrRowPtr; a fill
 // pass writes bsrColInd and the tile words (one coalesced store of b words).
+// The merge takes one step per tile, with the lanes of rows that miss the
+// tile idle, so slabs of more than a few entries go to k_pack_wide instead: a
+// block per slab, a thread per entry (see there).
 #include <vector>
 #include <algorithm>
 #include "graph.cuh"
@@ -34,19 +37,17 @@ __device__ __forceinline__ int seg_min(int v, int width) {
   return v;
 }
 
-// Per-lane cursor over one CSR row.
+// Per-lane cursor over one CSR row; head is the column at pos.
 struct RowCursor {
-  long long pos, end;
-  int prev;
+  int pos, end, head;
 };
 
-__device__ __forceinline__ void init_cursor(RowCursor& c, const int* __restrict__ rowptr, int row,
-                                            int nrows, long long nnz, unsigned* derr) {
+__device__ __forceinline__ void init_cursor(RowCursor& c, const int* __restrict__ rowptr, const int* __restrict__ colind,
+                                            int row, int nrows, long long nnz, unsigned* derr) {
   c.pos = 0;
   c.end = 0;
-  c.prev = -1;
   if (row < nrows) {
-    long long a = rowptr[row], e = rowptr[row + 1];
+    const int a = rowptr[row], e = rowptr[row + 1];
     if (a < 0 || e < a || e > nnz) {
       atomicOr(derr, DERR_ROWPTR);
     } else {
@@ -54,37 +55,88 @@ __device__ __forceinline__ void init_cursor(RowCursor& c, const int* __restrict_
       c.end = e;
     }
   }
+  c.head = c.pos < c.end ? colind[c.pos] : kINF;
 }
 
 template <int B>
-__device__ __forceinline__ int head_of(const RowCursor& c, const int* __restrict__ colind) {
-  return c.pos < c.end ? colind[c.pos] / B : kINF;
+__device__ __forceinline__ int head_block(const RowCursor& c) {
+  return c.pos < c.end ? c.head / B : kINF;
 }
 
-// Consume all entries of block column m from the cursor; OR their bits.
+// Consume all entries of block column m from the cursor; OR their bits.  An
+// entry below the one before it marks the row unsorted.
 template <int B, typename WT>
 __device__ __forceinline__ void consume(RowCursor& c, const int* __restrict__ colind, int m,
                                         int ncols, WT& word, unsigned* derr, bool build) {
-  while (c.pos < c.end) {
-    int col = colind[c.pos];
-    if (col / B != m) break;
-    if (col < c.prev) atomicOr(derr, DERR_UNSORTED);
+  while (c.pos < c.end && c.head / B == m) {
+    const int col = c.head;
     if (col < 0 || col >= ncols) atomicOr(derr, DERR_COL_BOUNDS);
-    c.prev = col;
     if (build) word |= (WT)((WT)1 << (B - 1 - ((unsigned)col % B)));
-    ++c.pos;
+    if (++c.pos >= c.end) break;
+    c.head = colind[c.pos];
+    if (c.head < col) atomicOr(derr, DERR_UNSORTED);
   }
 }
 
-// After a lane's row ends, any remaining (unsorted) entries are still
-// consumed by the merge; a head < previous column marks the row unsorted.
+// Which slabs go to k_pack_wide.  The merge takes a step per tile and, inside
+// it, a turn per entry of the longest run, so a slab is wide when it has more
+// than merge_tiles tiles or a row of more than kMergeRow entries.  The fill
+// pass knows the tiles; the count pass bounds them by the slab's entries
+// (kMergeEntries, which also keeps short slabs of long rows) and by the block
+// columns between its first and its last one.  k_pack asks and lists the
+// slab's units.
+// Measured (count and fill, us): the merge alone takes 24,700 on R-MAT 19
+// (16 edges a vertex, b = 32), where block row 0 alone has 16,384 tiles; wide
+// slabs past 48 / 64 / 96 tiles 662 / 660 / 696, and at b = 4 (1,138 / 989 /
+// 987, so 80 there).  Meshes (250 entries and 7 tiles a slab at b = 32) merge
+// in 92 and would take 185 as wide slabs; a dense 1,100-vertex R-MAT (35
+// tiles, rows of hundreds) merges in 231 and takes 144.  kMergeEntries 128 is
+// for b = 16 meshes (115; 173 at 64 entries) at the cost of 2 % on R-MAT.
+constexpr int kMergeEntries = 128;
+constexpr int kMergeRow = 48;
 template <int B>
-__device__ __forceinline__ void check_head(const RowCursor& c, const int* __restrict__ colind,
-                                           unsigned* derr) {
-  if (c.pos < c.end && c.prev >= 0 && colind[c.pos] < c.prev) atomicOr(derr, DERR_UNSORTED);
+__host__ __device__ constexpr int merge_tiles() {
+  return B == 4 ? 80 : 48;
+}
+constexpr int kUnitEntries = 2048;
+
+// Units of a slab with this many entries.
+__host__ __device__ __forceinline__ int units_of(long long entries) {
+  return entries <= 2 * kUnitEntries ? 1 : (int)((entries + kUnitEntries - 1) / kUnitEntries);
 }
 
-// COUNT (build=false) and FILL (build=true) share one body.
+struct __align__(16) WideUnit {
+  int slab, index, count, first;  // unit `index` of the slab's `count`, which start at unit `first`
+};
+
+// The units of the wide slabs, listed by k_pack and taken by k_pack_wide.
+struct WideList {
+  WideUnit* units = nullptr;          // null: no slab is wide
+  unsigned long long* ctr = nullptr;  // {units listed, taken, taken by the hubs' count}, zeroed by the caller
+  long long cap = 0;
+};
+
+// List a wide slab's units (one lane).  Row pointers that are not monotone
+// can ask for more than `cap`: those units get no slab.
+__device__ __forceinline__ void list_units(const WideList& wl, int slab, long long entries, long long nnz,
+                                           unsigned* derr) {
+  const int n = entries > nnz ? 0 : units_of(entries);
+  const unsigned long long first = atomicAdd(wl.ctr, (unsigned long long)n);
+  const bool fits = n > 0 && first + n <= (unsigned long long)wl.cap;
+  if (!fits) atomicOr(derr, DERR_ROWPTR);
+  for (int i = 0; i < n && first + i < (unsigned long long)wl.cap; ++i)
+    wl.units[first + i] = WideUnit{fits ? slab : -1, i, n, (int)first};
+}
+
+template <int B>
+__device__ __forceinline__ long long slab_entries(const int* __restrict__ rowptr, long long slab, int nrows) {
+  const long long a = slab * B, e = a + B < nrows ? a + B : nrows;
+  return (long long)rowptr[e] - (long long)rowptr[a];
+}
+
+// COUNT (build=false) and FILL (build=true) share one body.  A wide slab is
+// listed for k_pack_wide and left alone (its count starts at zero: its units
+// add to it).
 template <int B, bool BUILD>
 __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowptr,
                                                    const int* __restrict__ colind, int nrows,
@@ -93,7 +145,7 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
                                                    const int* __restrict__ bsr_rowptr,
                                                    int* __restrict__ bsr_colind,
                                                    typename Word<B>::T* __restrict__ bsr_val,
-                                                   int layout, unsigned* derr) {
+                                                   int layout, WideList wl, unsigned* derr) {
   using WT = typename Word<B>::T;
   using M = SlabMap<B>;
   const unsigned lane = threadIdx.x & 31;
@@ -102,38 +154,71 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
   const int r = lane % M::W;          // row within slab (first row for B=64)
   const long long slab = warp * M::G + g;
   if (warp * M::G >= nbr) return;     // whole warp idle (uniform)
-  const bool slab_ok = slab < nbr;
+  bool slab_ok = slab < nbr;
 
   RowCursor c0, c1;
   const long long row0 = slab * B + r;
-  init_cursor(c0, rowptr, slab_ok && row0 < nrows ? (int)row0 : nrows, nrows, nnz, derr);
+  init_cursor(c0, rowptr, colind, slab_ok && row0 < nrows ? (int)row0 : nrows, nrows, nnz, derr);
   if (M::RPL == 2) {
     const long long row1 = slab * B + 32 + r;
-    init_cursor(c1, rowptr, slab_ok && row1 < nrows ? (int)row1 : nrows, nrows, nnz, derr);
+    init_cursor(c1, rowptr, colind, slab_ok && row1 < nrows ? (int)row1 : nrows, nrows, nnz, derr);
+  }
+  if (wl.units) {
+    const long long entries = slab_ok ? slab_entries<B>(rowptr, slab, nrows) : 0;
+    int longest = c0.end - c0.pos;
+    if (M::RPL == 2) longest = max(longest, c1.end - c1.pos);
+    longest = -seg_min(-longest, M::W);
+    bool w = slab_ok && entries > kMergeEntries;
+    if (BUILD) {
+      w = slab_ok && (bsr_rowptr[slab + 1] - bsr_rowptr[slab] > merge_tiles<B>() || longest > kMergeRow);
+    } else if (__any_sync(0xffffffffu, w)) {
+      int first = c0.head, last = c0.pos < c0.end ? colind[c0.end - 1] : -1;
+      if (M::RPL == 2) {
+        first = min(first, c1.head);
+        last = max(last, c1.pos < c1.end ? colind[c1.end - 1] : -1);
+      }
+      first = seg_min(first, M::W);
+      last = -seg_min(-last, M::W);
+      w = w && (longest > kMergeRow || (long long)last / B - (long long)first / B >= merge_tiles<B>());
+    }
+    if (w) {
+      if (r == 0) {
+        if (!BUILD) counts[slab] = 0;
+        list_units(wl, (int)slab, entries, nnz, derr);
+      }
+      slab_ok = false;
+      c0.end = c0.pos;
+      if (M::RPL == 2) c1.end = c1.pos;
+    }
+    if (!__any_sync(0xffffffffu, slab_ok)) return;
   }
 
+  // a slab's tiles stay inside its block row's range of the output
   long long out = 0;
-  if (BUILD && slab_ok) out = bsr_rowptr[slab];
+  int room = 0;
+  if (BUILD && slab_ok) {
+    out = bsr_rowptr[slab];
+    room = (int)(bsr_rowptr[slab + 1] - out);
+  }
   int ntile = 0;
 
   while (true) {
-    int h = head_of<B>(c0, colind);
-    if (M::RPL == 2) h = min(h, head_of<B>(c1, colind));
+    int h = head_block<B>(c0);
+    if (M::RPL == 2) h = min(h, head_block<B>(c1));
     const int m = seg_min(h, M::W);
     if (!__any_sync(0xffffffffu, m != kINF)) break;
     WT w0 = 0, w1 = 0;
     if (m != kINF) {
       consume<B, WT>(c0, colind, m, ncols, w0, derr, BUILD);
-      check_head<B>(c0, colind, derr);
       if (M::RPL == 2) {
         consume<B, WT>(c1, colind, m, ncols, w1, derr, BUILD);
-        check_head<B>(c1, colind, derr);
       }
     }
     if (BUILD) {
       const long long tile = out + ntile;
+      const bool put = m != kINF && ntile < room;
       if (layout == GBO_LAYOUT_ROW) {
-        if (m != kINF) {
+        if (put) {
           if (r == 0) bsr_colind[tile] = m;
           bsr_val[tile * B + r] = w0;
           if (M::RPL == 2) bsr_val[tile * B + 32 + r] = w1;
@@ -150,7 +235,7 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
             unsigned colw = __brev(seg) >> (32 - (B < 32 ? B : 32));
             if (r == cc) mine = (WT)colw;
           }
-          if (m != kINF) {
+          if (put) {
             if (r == 0) bsr_colind[tile] = m;
             bsr_val[tile * B + r] = mine;
           }
@@ -164,7 +249,7 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
             if (cc == (int)r) lo_w = colw;
             if (cc == (int)r + 32) hi_w = colw;
           }
-          if (m != kINF) {
+          if (put) {
             if (r == 0) bsr_colind[tile] = m;
             bsr_val[tile * B + r] = (WT)lo_w;
             bsr_val[tile * B + 32 + r] = (WT)hi_w;
@@ -175,6 +260,315 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
     if (m != kINF) ++ntile;
   }
   if (!BUILD && slab_ok && r == 0) counts[slab] = ntile;
+}
+
+// Wide slabs.  A block takes a unit: a whole slab or, of a hub slab, the
+// block columns between two quantiles of its longest row, about kUnitEntries
+// entries.  A thread per row finds the row's entries in the unit (binary
+// search); the block walks these with a thread per entry, four in flight,
+// and marks their block columns in a shared-memory bitmap, whose set bits are
+// the unit's tiles in order.  The count pass adds up the newly set bits.  The
+// fill pass ranks the bitmap (per-warp prefix sums of the words' popcounts),
+// writes bsrColInd, zeroes the unit's tiles and walks the entries again: in
+// the ROW layout the first entry of a run (entries of one row in one block
+// column are consecutive) gathers the run's bits and stores the whole row
+// word, in the COL layout an entry ORs its bit into its column word.  Block
+// columns past the bitmap's `win` are taken in further windows.
+//
+// What bounds it: the tile writes (a 32x32 tile is 128 bytes for one or two
+// row words on power-law graphs); a unit's tiles are zeroed just before their
+// words are stored so that both meet in L2.  R-MAT 19, b = 32 (1.4 GB of
+// tiles): 357 us for the fill and 107 for the count.  One block of 1,024
+// threads per hub slab instead of units: 666 (block row 0 is the tail);
+// tiles built in shared memory by a lane per row: 2,000 (serial walks); all
+// tiles zeroed by a kernel of their own first: 15 % more.
+constexpr int kWideTPB = 128;
+constexpr int kWideWarps = kWideTPB / 32;
+constexpr int kWideInFlight = 4;
+constexpr int kWideBlocksPerSM = 16;
+constexpr size_t kWideShared = 224 * 1024;  // dynamic shared memory of a block, at most (227 KB less the static arrays)
+
+// Inclusive sums of the values v[1..B] in place (v[0] = 0), by one warp.
+template <int B>
+__device__ __forceinline__ void warp_prefix_rows(int* v, unsigned lane) {
+  int carry = 0;
+#pragma unroll
+  for (int h = 0; h < (B + 31) / 32; ++h) {
+    const int i = (int)lane + 32 * h;
+    int x = i < B ? v[i + 1] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if ((int)lane >= o) x += y;
+    }
+    x += carry;
+    if (i < B) v[i + 1] = x;
+    carry = __shfl_sync(0xffffffffu, x, 31);
+  }
+  if (lane == 0) v[0] = 0;
+}
+
+// `split_only`: the units of hub slabs alone (their counts, ahead of the fill
+// pass).  ucnt: tiles of every unit -- written by the count form, summed by
+// the fill form into its first tile.
+template <int B, bool BUILD>
+__global__ void __launch_bounds__(kWideTPB) k_pack_wide(const int* __restrict__ rowptr,
+                                                        const int* __restrict__ colind, int nrows, int ncols,
+                                                        long long nnz, int nbc, int win,
+                                                        WideList wl, bool split_only, int* ucnt, int* __restrict__ counts,
+                                                        const int* __restrict__ bsr_rowptr,
+                                                        int* __restrict__ bsr_colind,
+                                                        typename Word<B>::T* bsr_val, int layout,
+                                                        unsigned* derr) {
+  using WT = typename Word<B>::T;
+  constexpr int F = kWideInFlight;
+  extern __shared__ unsigned wide_sh[];
+  __shared__ int rp[B + 1], seg_beg[B], seg_pre[B + 1];  // rows' entries: all, the window's first, the window's count before
+  __shared__ int longest_sh;
+  __shared__ unsigned long long unit_sh;
+  __shared__ int wsum[kWideWarps + 1];
+  const int nwords = win / 32;
+  unsigned* bm = wide_sh;                               // block column w0 + 32 i + k: bit k of word i
+  int* pre = reinterpret_cast<int*>(wide_sh + nwords);  // BUILD: tiles before word i within its warp's range
+  const int tid = (int)threadIdx.x;
+  const unsigned lane = threadIdx.x & 31;
+  const int wib = tid >> 5;
+  const int shift = nwords <= kWideWarps ? 0 : 32 - __clz((nwords - 1) / kWideWarps);
+  const int per_warp = 1 << shift;  // words ranked by one warp
+  const unsigned long long nunits = min(wl.ctr[0], (unsigned long long)wl.cap);
+  for (;;) {
+    __syncthreads();  // the previous unit's readers of the shared arrays
+    if (tid == 0) unit_sh = atomicAdd(wl.ctr + (split_only ? 2 : 1), 1ull);
+    __syncthreads();
+    if (unit_sh >= nunits) return;
+    const int ui = (int)unit_sh;
+    const WideUnit un = wl.units[ui];
+    if (un.slab < 0 || (split_only && un.count == 1)) continue;
+    const long long row0 = (long long)un.slab * B;
+    const int rows = (int)(row0 + B < nrows ? B : nrows - row0);
+    if (tid <= rows) rp[tid] = rowptr[row0 + tid];
+    __syncthreads();
+    const bool bad = tid < rows && (rp[tid] < 0 || rp[tid + 1] < rp[tid] || rp[tid + 1] > nnz);
+    if (__syncthreads_or(bad)) {
+      if (tid == 0) {
+        atomicOr(derr, DERR_ROWPTR);
+        if (!BUILD && ucnt) ucnt[ui] = 0;
+      }
+      continue;
+    }
+    long long wa = 0, wz = nbc;  // the unit's block columns
+    if (un.count > 1) {
+      if (wib == 0) {  // the longest row
+        int len = -1, at = 0;
+        for (int r = (int)lane; r < rows; r += 32)
+          if (rp[r + 1] - rp[r] > len) {
+            len = rp[r + 1] - rp[r];
+            at = r;
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const int l2 = __shfl_xor_sync(0xffffffffu, len, o), a2 = __shfl_xor_sync(0xffffffffu, at, o);
+          if (l2 > len || (l2 == len && a2 < at)) {
+            len = l2;
+            at = a2;
+          }
+        }
+        if (lane == 0) longest_sh = at;
+      }
+      __syncthreads();
+      const int b0 = rp[longest_sh];
+      const long long len = rp[longest_sh + 1] - b0;
+      if (un.index > 0) wa = min((long long)max(colind[b0 + len * un.index / un.count], 0) / B, (long long)nbc);
+      if (un.index + 1 < un.count)
+        wz = min((long long)max(colind[b0 + len * (un.index + 1) / un.count], 0) / B, (long long)nbc);
+      if (!BUILD) {
+        // this unit's share of the slab's entries checked one by one (the
+        // rows' searches below suppose them sorted)
+        const int e0 = rp[0];
+        const long long ne = rp[rows] - e0;
+        const long long ez = e0 + ne * (un.index + 1) / un.count;
+        for (long long e = e0 + ne * un.index / un.count + tid; e < ez; e += kWideTPB) {
+          const int c = colind[e];
+          if (c < 0 || c >= ncols) atomicOr(derr, DERR_COL_BOUNDS);
+          if (e > e0 && c < colind[e - 1]) {
+            bool starts = false;
+            for (int r = 0; r < rows; ++r) starts = starts || rp[r] == (int)e;
+            if (!starts) atomicOr(derr, DERR_UNSORTED);
+          }
+        }
+      }
+    }
+    long long t0 = 0, t1 = 0;
+    if (BUILD) {
+      t0 = bsr_rowptr[un.slab];
+      t1 = bsr_rowptr[un.slab + 1];
+      if (un.index > 0) {  // behind the tiles of the slab's earlier units
+        int v = 0;
+        for (int i = tid; i < un.index; i += kWideTPB) v += ucnt[un.first + i];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) wsum[wib] = v;
+        __syncthreads();
+        for (int q = 0; q < kWideWarps; ++q) t0 += wsum[q];
+        __syncthreads();
+      }
+    }
+    int cnt = 0;
+    for (long long w0 = wa; w0 < wz; w0 += win) {
+      const long long w1 = min(w0 + win, wz);
+      const int nw = (int)((w1 - w0 + 31) / 32);  // bitmap words in use
+      __syncthreads();
+      for (int i = tid; i < nw; i += kWideTPB) bm[i] = 0u;
+      if (tid < B) {
+        int lo = 0, hi = 0;
+        if (tid < rows) {
+          lo = rp[tid];
+          hi = rp[tid + 1];
+          if (w0 > 0 || w1 < nbc) {
+            int top = hi;
+            while (lo < hi) {  // first entry at or past block column w0
+              const int mid = (lo + hi) >> 1;
+              if (colind[mid] < w0 * B) lo = mid + 1;
+              else hi = mid;
+            }
+            while (hi < top) {  // first entry at or past block column w1
+              const int mid = (hi + top) >> 1;
+              if (colind[mid] < w1 * B) hi = mid + 1;
+              else top = mid;
+            }
+          }
+        }
+        seg_beg[tid] = lo;
+        seg_pre[tid + 1] = hi - lo;
+      }
+      __syncthreads();
+      if (wib == 0) warp_prefix_rows<B>(seg_pre, lane);
+      __syncthreads();
+      const int ne = seg_pre[B];
+      // entry q of the window: its row, place, column and the column before it in its row (-1: none)
+      auto entry = [&](int q, int& r, int& e, int& c, int& cp) {
+        c = cp = -1;
+        if (q >= ne) return;
+        r = 0;
+#pragma unroll
+        for (int st = B / 2; st > 0; st >>= 1)
+          if (seg_pre[r + st] <= q) r += st;
+        e = seg_beg[r] + (q - seg_pre[r]);
+        c = colind[e];
+        if (e > rp[r]) cp = colind[e - 1];
+      };
+      for (int qb = tid; qb < ne; qb += kWideTPB * F) {
+        int r[F], e[F], c[F], cp[F];
+#pragma unroll
+        for (int u = 0; u < F; ++u) entry(qb + u * kWideTPB, r[u], e[u], c[u], cp[u]);
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+          if (qb + u * kWideTPB >= ne) break;
+          if (c[u] < 0 || c[u] >= ncols) {
+            atomicOr(derr, DERR_COL_BOUNDS);
+            continue;
+          }
+          if (c[u] < cp[u]) atomicOr(derr, DERR_UNSORTED);
+          const int C = c[u] / B;
+          if (cp[u] >= 0 && cp[u] / B == C) continue;  // marked by the entry before
+          const long long k = C - w0;
+          if (k < 0 || C >= w1) continue;  // an unsorted row's
+          const unsigned bit = 1u << (k & 31);
+          if (!(*(volatile unsigned*)(bm + (k >> 5)) & bit) && !(atomicOr(bm + (k >> 5), bit) & bit)) ++cnt;
+        }
+      }
+      if (!BUILD) continue;
+      __syncthreads();
+      // rank: every warp over its own range of words, then the warps' totals
+      const int i0 = wib << shift, i1 = min(i0 + per_warp, nw);
+      int run = 0;
+      for (int i = i0; i < i1; i += 32) {
+        const int p = i + (int)lane < i1 ? __popc(bm[i + lane]) : 0;
+        int incl = p;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if ((int)lane >= o) incl += y;
+        }
+        if (i + (int)lane < i1) pre[i + lane] = run + incl - p;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) wsum[wib + 1] = run;
+      __syncthreads();
+      if (wib == 0) {
+        int v = lane < kWideWarps ? wsum[lane + 1] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, v, o);
+          if ((int)lane >= o) v += y;
+        }
+        if (lane < kWideWarps) wsum[lane + 1] = v;
+        if (lane == 0) wsum[0] = 0;
+      }
+      __syncthreads();
+      const long long tz = min(t1, t0 + wsum[kWideWarps]);  // a slab's tiles stay inside its range of the output
+      for (int i = i0 + (int)lane; i < i1; i += 32) {
+        long long t = t0 + wsum[wib] + pre[i];
+        for (unsigned m = bm[i]; m; m &= m - 1, ++t)
+          if (t < tz) bsr_colind[t] = (int)(w0 + 32 * i + (__ffs(m) - 1));
+      }
+      {
+        constexpr int kTileWords = B * (int)sizeof(WT) / 4;
+        unsigned* z = reinterpret_cast<unsigned*>(bsr_val) + t0 * kTileWords;
+        const long long nz = (tz - t0) * kTileWords;
+        if (kTileWords % 4 == 0 && reinterpret_cast<uintptr_t>(bsr_val) % 16 == 0)
+          for (long long i = tid; i < nz / 4; i += kWideTPB) reinterpret_cast<uint4*>(z)[i] = make_uint4(0u, 0u, 0u, 0u);
+        else
+          for (long long i = tid; i < nz; i += kWideTPB) z[i] = 0u;
+      }
+      __syncthreads();
+      for (int qb = tid; qb < ne; qb += kWideTPB * F) {
+        int r[F], e[F], c[F], cp[F];
+#pragma unroll
+        for (int u = 0; u < F; ++u) entry(qb + u * kWideTPB, r[u], e[u], c[u], cp[u]);
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+          if (c[u] < 0 || c[u] >= ncols) continue;  // past the end, or reported above
+          const int C = c[u] / B;
+          if (C < w0 || C >= w1) continue;
+          if (layout == GBO_LAYOUT_ROW && cp[u] >= 0 && cp[u] / B == C) continue;  // inside its run
+          const int k = (int)(C - w0);
+          const long long t = t0 + wsum[k >> (shift + 5)] + pre[k >> 5] + __popc(bm[k >> 5] & ((1u << (k & 31)) - 1u));
+          if (t >= tz) continue;
+          if (layout == GBO_LAYOUT_ROW) {
+            WT word = (WT)((WT)1 << (B - 1 - c[u] % B));
+            for (int f = e[u] + 1; f < rp[r[u] + 1]; ++f) {
+              const int cf = colind[f];
+              if (cf < 0 || cf / B != C) break;
+              word = (WT)(word | ((WT)1 << (B - 1 - cf % B)));
+            }
+            bsr_val[t * B + r[u]] = word;
+          } else {
+            const long long wi = t * B + c[u] % B;
+            if constexpr (B == 64) {
+              atomicOr(reinterpret_cast<unsigned long long*>(bsr_val) + wi, 1ull << (B - 1 - r[u]));
+            } else {
+              constexpr int kPer = 4 / (int)sizeof(WT);  // words of a 32-bit atomic (little endian)
+              atomicOr(reinterpret_cast<unsigned*>(bsr_val) + wi / kPer,
+                       (1u << (B - 1 - r[u])) << ((wi % kPer) * 8 * (int)sizeof(WT)));
+            }
+          }
+        }
+      }
+      t0 = tz;
+      __syncthreads();  // wsum is rewritten
+    }
+    if (!BUILD) {
+      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+      if (lane == 0) wsum[wib] = cnt;
+      __syncthreads();
+      if (tid == 0) {
+        int tot = 0;
+        for (int q = 0; q < kWideWarps; ++q) tot += wsum[q];
+        if (ucnt) ucnt[ui] = tot;
+        if (counts && tot) atomicAdd(counts + un.slab, tot);
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------- scan
@@ -229,6 +623,41 @@ __global__ void k_scan_sums(long long* __restrict__ sums, long long nb, long lon
     __syncthreads();
   }
   if (threadIdx.x == 0) *total = carry;
+}
+
+// Short inputs (kScanShort): one kernel, every block adding up the counts of
+// the blocks before it itself -- at most 15 coalesced loads a thread, where
+// the three kernels above cost three launches (16,384 counts: 7 us of kernels, 10 as three).
+constexpr long long kScanShort = 16 * kScanTPB;
+
+template <typename OutT>
+__global__ void __launch_bounds__(kScanTPB) k_scan_short(const int* __restrict__ in, int n, OutT* __restrict__ out,
+                                                         long long* __restrict__ total) {
+  __shared__ long long sh[32], base_sh[32];
+  const unsigned lane = threadIdx.x & 31;
+  const int w = (int)(threadIdx.x >> 5);
+  const int i = (int)blockIdx.x * kScanTPB + (int)threadIdx.x;
+  long long before = 0;
+#pragma unroll 8
+  for (int k = (int)threadIdx.x; k < (int)blockIdx.x * kScanTPB; k += kScanTPB) before += in[k];
+  const long long v = i < n ? in[i] : 0;
+  long long x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if ((int)lane >= o) x += y;
+  }
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 31) sh[w] = x;
+  if (lane == 0) base_sh[w] = before;
+  __syncthreads();
+  long long base = 0;
+  for (int q = 0; q < kScanTPB / 32; ++q) base += base_sh[q] + (q < w ? sh[q] : 0);
+  const long long excl = base + x - v, most = sizeof(OutT) == 8 ? excl : 2147483647LL;
+  if (i < n) out[i] = (OutT)min(excl, most);
+  if (i == n - 1) {
+    out[n] = (OutT)min(excl + v, sizeof(OutT) == 8 ? excl + v : 2147483647LL);
+    *total = excl + v;
+  }
 }
 
 template <typename OutT>
@@ -360,36 +789,81 @@ __global__ void k_sched_fill(const int* __restrict__ rowptr, int nbr, int chunk,
   }
 }
 
+// Block columns of k_pack_wide's bitmap: all of them, as far as their words
+// and the words' ranks (8 bytes for 32 block columns) fit a block.
+int wide_window(int nbc) {
+  const long long all = ((long long)nbc + 1023) / 1024 * 1024;
+  return (int)std::max(1024ll, std::min(all, (long long)(kWideShared / 8) / 32 * 1024));
+}
+
+template <int B, bool BUILD>
+int launch_pack_pass(const int* rowptr, const int* colind, int nrows, int ncols, long long nnz, int nbr, int* counts,
+                     const int* bsr_rowptr, int* bsr_colind, typename Word<B>::T* bsr_val, int layout,
+                     unsigned* derr, unsigned long long* ctr, cudaStream_t s) {
+  using M = SlabMap<B>;
+  const long long warps = ((long long)nbr + M::G - 1) / M::G;
+  const unsigned grid = blocks_for_warps(warps, kPackTPB / 32);
+  // entries of a wide slab, at least (a tile or a row's entry each)
+  constexpr int kLeast = merge_tiles<B>() < kMergeRow ? merge_tiles<B>() : kMergeRow;
+  // the wide kernel stores the tile array in whole 32-bit words
+  const bool wide = nnz > kLeast && (!BUILD || reinterpret_cast<uintptr_t>(bsr_val) % 4 == 0);
+  WideList wl;
+  int* ucnt = nullptr;
+  char* tmp = nullptr;  // the units and (fill pass) their tile counts
+  if (wide) {
+    const long long slabs = std::min<long long>(nbr, nnz / (kLeast + 1));
+    wl.cap = std::max(slabs + nnz / kUnitEntries, 1ll);
+    wl.ctr = ctr;
+    const size_t unit_bytes = sizeof(WideUnit) * (size_t)wl.cap;
+    GBO_CUDA_TRY(pool_malloc_async(&tmp, unit_bytes + (BUILD ? sizeof(int) * (size_t)wl.cap : 0), s));
+    wl.units = reinterpret_cast<WideUnit*>(tmp);
+    if (BUILD) ucnt = reinterpret_cast<int*>(tmp + unit_bytes);
+  }
+  k_pack<B, BUILD><<<grid, kPackTPB, 0, s>>>(rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind,
+                                             bsr_val, layout, wl, derr);
+  int st = GBO_OK;
+  if (wide) {
+    const int nbc = (ncols + B - 1) / B;
+    const int win = wide_window(nbc);
+    const unsigned blocks = (unsigned)std::min<long long>(wl.cap, (long long)num_sms() * kWideBlocksPerSM);
+    auto launch = [&](auto kern, size_t smem, bool split_only) -> int {
+      if (smem > 40 * 1024)
+        GBO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideShared));
+      kern<<<blocks, kWideTPB, smem, s>>>(rowptr, colind, nrows, ncols, nnz, nbc, win, wl, split_only, ucnt, counts,
+                                          bsr_rowptr, bsr_colind, bsr_val, layout, derr);
+      return GBO_OK;
+    };
+    const size_t bits = (size_t)win / 8;
+    // fill: the hub units' tile counts first
+    if (!BUILD || nnz > 2 * kUnitEntries) st = launch(k_pack_wide<B, false>, bits, BUILD);
+    if (BUILD && st == GBO_OK) st = launch(k_pack_wide<B, true>, 2 * bits, false);
+  }
+  const cudaError_t e = cudaGetLastError();
+  if (tmp) cudaFreeAsync(tmp, s);
+  if (e != cudaSuccess) return fail_cuda(e, "pack kernels");
+  return st;
+}
+
 template <int B>
 int launch_pack(bool build, const int* rowptr, const int* colind, int nrows, int ncols,
                 long long nnz, int nbr, int* counts, const int* bsr_rowptr, int* bsr_colind,
-                void* bsr_val, int layout, unsigned* derr, cudaStream_t s) {
-  using M = SlabMap<B>;
-  long long warps = (nbr + M::G - 1) / M::G;
-  unsigned grid = blocks_for_warps(warps, kPackTPB / 32);
-  if (build)
-    k_pack<B, true><<<grid, kPackTPB, 0, s>>>(rowptr, colind, nrows, ncols, nnz, nbr, counts,
-                                              bsr_rowptr, bsr_colind,
-                                              reinterpret_cast<typename Word<B>::T*>(bsr_val),
-                                              layout, derr);
-  else
-    k_pack<B, false><<<grid, kPackTPB, 0, s>>>(rowptr, colind, nrows, ncols, nnz, nbr, counts,
-                                               bsr_rowptr, bsr_colind,
-                                               reinterpret_cast<typename Word<B>::T*>(bsr_val),
-                                               layout, derr);
-  GBO_CUDA_TRY(cudaGetLastError());
-  return GBO_OK;
+                void* bsr_val, int layout, unsigned* derr, unsigned long long* ctr, cudaStream_t s) {
+  auto* val = reinterpret_cast<typename Word<B>::T*>(bsr_val);
+  return build ? launch_pack_pass<B, true>(rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, val,
+                                           layout, derr, ctr, s)
+               : launch_pack_pass<B, false>(rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind,
+                                            val, layout, derr, ctr, s);
 }
 
 int dispatch_pack(int b, bool build, const int* rowptr, const int* colind, int nrows, int ncols,
                   long long nnz, int nbr, int* counts, const int* bsr_rowptr, int* bsr_colind,
-                  void* bsr_val, int layout, unsigned* derr, cudaStream_t s) {
+                  void* bsr_val, int layout, unsigned* derr, unsigned long long* ctr, cudaStream_t s) {
   switch (b) {
-    case 4: return launch_pack<4>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, s);
-    case 8: return launch_pack<8>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, s);
-    case 16: return launch_pack<16>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, s);
-    case 32: return launch_pack<32>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, s);
-    case 64: return launch_pack<64>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, s);
+    case 4: return launch_pack<4>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, ctr, s);
+    case 8: return launch_pack<8>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, ctr, s);
+    case 16: return launch_pack<16>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, ctr, s);
+    case 32: return launch_pack<32>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, ctr, s);
+    case 64: return launch_pack<64>(build, rowptr, colind, nrows, ncols, nnz, nbr, counts, bsr_rowptr, bsr_colind, bsr_val, layout, derr, ctr, s);
   }
   return fail(GBO_ERR_INVALID, "tile_bits must be 4, 8, 16, 32 or 64");
 }
@@ -401,11 +875,12 @@ int derr_to_status(unsigned e) {
   return GBO_OK;
 }
 
-// Small device scratch for the scan + error word, stream-ordered.
-struct ScanScratch {
-  long long* sums = nullptr;
-  long long* total = nullptr;
-  unsigned* derr = nullptr;
+// A packing pass's device record, zeroed before it: the tile count, the
+// counters of the wide units (WideList::ctr) and the error word.
+struct PackRecord {
+  long long total;
+  unsigned long long units[3];
+  unsigned derr;
 };
 
 }  // namespace
@@ -415,6 +890,11 @@ template <typename OutT>
 int exclusive_scan(const int* d_in, OutT* d_out, long long n, long long* d_total, cudaStream_t s) {
   long long nb = (n + kScanTPB - 1) / kScanTPB;
   if (nb < 1) nb = 1;
+  if (n > 0 && n <= kScanShort) {
+    k_scan_short<OutT><<<(unsigned)nb, kScanTPB, 0, s>>>(d_in, (int)n, d_out, d_total);
+    GBO_CUDA_TRY(cudaGetLastError());
+    return GBO_OK;
+  }
   long long* sums = nullptr;
   GBO_CUDA_TRY(pool_malloc_async(&sums, sizeof(long long) * nb, s));
   k_scan_block_sums<<<(unsigned)nb, kScanTPB, 0, s>>>(d_in, n, sums);
@@ -442,34 +922,28 @@ static int nnzb_impl(const int* rowptr, const int* colind, int nrows, int ncols,
                      int b, int* bsr_rowptr, long long* h_total, cudaStream_t s) {
   const int nbr = (nrows + b - 1) / b;
   int* counts = nullptr;
-  long long* d_total = nullptr;
-  unsigned* derr = nullptr;
+  PackRecord* rec = nullptr;
   GBO_CUDA_TRY(pool_malloc_async(&counts, sizeof(int) * (size_t)(nbr > 0 ? nbr : 1), s));
-  GBO_CUDA_TRY(pool_malloc_async(&d_total, sizeof(long long) + sizeof(unsigned) * 2, s));
-  derr = reinterpret_cast<unsigned*>(d_total + 1);
-  GBO_CUDA_TRY(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
+  GBO_CUDA_TRY(pool_malloc_async(&rec, sizeof(PackRecord), s));
+  GBO_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(PackRecord), s));
   int st = GBO_OK;
   if (nbr > 0) {
     st = dispatch_pack(b, false, rowptr, colind, nrows, ncols, nnz, nbr, counts, nullptr, nullptr,
-                       nullptr, GBO_LAYOUT_ROW, derr, s);
-    if (st == GBO_OK) st = exclusive_scan_i32(counts, bsr_rowptr, nbr, d_total, s);
+                       nullptr, GBO_LAYOUT_ROW, &rec->derr, rec->units, s);
+    if (st == GBO_OK) st = exclusive_scan_i32(counts, bsr_rowptr, nbr, &rec->total, s);
   } else {
     GBO_CUDA_TRY(cudaMemsetAsync(bsr_rowptr, 0, sizeof(int), s));
-    GBO_CUDA_TRY(cudaMemsetAsync(d_total, 0, sizeof(long long), s));
   }
-  long long tot = 0;
-  unsigned herr = 0;
+  PackRecord h = {};
   if (st == GBO_OK) {
-    cudaError_t e1 = cudaMemcpyAsync(&tot, d_total, sizeof(long long), cudaMemcpyDeviceToHost, s);
-    cudaError_t e2 = cudaMemcpyAsync(&herr, derr, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    cudaError_t e3 = cudaStreamSynchronize(s);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
-      st = fail_cuda(e3 != cudaSuccess ? e3 : (e1 != cudaSuccess ? e1 : e2), "nnzb readback");
+    const cudaError_t e = read_back(&h, rec, sizeof(h), s);
+    if (e != cudaSuccess) st = fail_cuda(e, "nnzb readback");
   }
+  const long long tot = h.total;
   cudaFreeAsync(counts, s);
-  cudaFreeAsync(d_total, s);
+  cudaFreeAsync(rec, s);
   if (st != GBO_OK) return st;
-  GBO_TRY(derr_to_status(herr));
+  GBO_TRY(derr_to_status(h.derr));
   if (tot > 2147483647LL) return fail(GBO_ERR_OVERFLOW, "more than 2^31-1 tiles; use a wider tile");
   *h_total = tot;
   return GBO_OK;
@@ -492,18 +966,17 @@ static int fill_impl(const int* rowptr, const int* colind, int nrows, int ncols,
                      cudaStream_t s, bool check) {
   const int nbr = (nrows + b - 1) / b;
   if (nbr == 0) return GBO_OK;
-  unsigned* derr = nullptr;
-  GBO_CUDA_TRY(pool_malloc_async(&derr, sizeof(unsigned), s));
-  GBO_CUDA_TRY(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
+  PackRecord* rec = nullptr;
+  GBO_CUDA_TRY(pool_malloc_async(&rec, sizeof(PackRecord), s));
+  GBO_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(PackRecord), s));
   int st = dispatch_pack(b, true, rowptr, colind, nrows, ncols, nnz, nbr, nullptr, bsr_rowptr,
-                         bsr_colind, bsr_val, layout, derr, s);
+                         bsr_colind, bsr_val, layout, &rec->derr, rec->units, s);
   unsigned herr = 0;
   if (st == GBO_OK && check) {
-    cudaError_t e1 = cudaMemcpyAsync(&herr, derr, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    cudaError_t e2 = cudaStreamSynchronize(s);
-    if (e1 != cudaSuccess || e2 != cudaSuccess) st = fail_cuda(e1 != cudaSuccess ? e1 : e2, "pack");
+    const cudaError_t e = read_back(&herr, &rec->derr, sizeof(herr), s);
+    if (e != cudaSuccess) st = fail_cuda(e, "pack");
   }
-  cudaFreeAsync(derr, s);
+  cudaFreeAsync(rec, s);
   if (st != GBO_OK) return st;
   return derr_to_status(herr);
 }
