@@ -260,15 +260,6 @@ def bfs_level_bytes_rws(csr, levels, head=8):
     return out
 
 
-def row_word_counts(csr, b=32):
-    """Non-empty b-bit row words of every row: its distinct block columns."""
-    prow = np.repeat(np.arange(csr.nrows, dtype=np.int64), np.diff(csr.rowptr))
-    pcol = (csr.colind // b).astype(np.int64)
-    first = np.ones(len(pcol), bool)
-    first[1:] = (pcol[1:] != pcol[:-1]) | (prow[1:] != prow[:-1])
-    return np.bincount(prow[first], minlength=csr.nrows).astype(np.int64)
-
-
 def load_peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -1085,24 +1076,17 @@ def suite_config2(args, which):
                     args.steps, args.warmup)
         st = g.last_run()
         step = float(np.mean(st["step_ms"])) if st["step_ms"] else ms / iters
-        if args.tile == 32:
-            # row-word slices: every non-empty row word once with its block
-            # column (8 bytes), the tail offsets of rows past the head, and
-            # per vertex the iterate read, its 1/deg, and the two outputs
-            # written (16 bytes); the gathered p/deg words are excluded (a
-            # 16 MB vector that L2 holds)
-            words = row_word_counts(csr)
-            by = 8 * int(words.sum()) + 16 * int(np.count_nonzero(words > 8)) + 16 * n
-            kname = "k_pr_step_rws (PageRank iteration over row-word slices)"
-        else:
-            by = _bmv_bytes(info, args.tile, n, 4 * n * 5)  # p/deg gathered, p, D^-1 read; p', p'/deg written
-            kname = "k_pr_step (PageRank iteration, semiring BMV + update)"
+        # the row lists: every set bit's column once (4 bytes), the row offsets,
+        # and per vertex the iterate read, its 1/deg, and the two outputs
+        # written (16 bytes); the gathered p/deg words are excluded (a vector
+        # that L2 holds)
+        by = 4 * csr.nnz + 8 * (n + 1) + 16 * n
+        kname = "k_pr_loop (one PageRank iteration of the cooperative launch)"
         cfg["workload"] = f"PageRank alpha 0.85, 20 iterations, fp32 values / fp64 sums, R-MAT scale {args.scale}"
         extra = {"iterations": it.value, "dtype": "f32",
                  "roofline": {"bound": "hbm", "achieved": by / (step / 1e3) / 1e9, "peak": peak,
                               "unit": "GB/s", "frac": by / (step / 1e3) / 1e9 / peak,
-                              "traffic": (load_traffic("k_pr_step_rws_rmat20_ncu.md", by)
-                                          if args.tile == 32 else None),
+                              "traffic": load_traffic("k_pr_loop_rmat20_ncu.md", by),
                               "kernel": kname, "peak_source": psrc,
                               "algorithmic_bytes_per_launch": by, "ms_per_launch": step}}
         if bs is not None:

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "gather.cuh"
 #include "scan.cuh"
 
 namespace gbo {
@@ -46,6 +47,7 @@ struct Ctrl {
   // new-vertex counts of three consecutive levels
   unsigned bar_arrive;
   unsigned bar_err;
+  double err_part[3][8][16];       // errors of three consecutive PageRank iterations, spread as lvl_part
   unsigned long long push_acc[3];  // push list: rows << 40 | tail entries
   // new-vertex counts of three consecutive levels, each spread over eight
   // counters on their own 128-byte lines (block b adds into counter b % 8)
@@ -78,7 +80,7 @@ struct AlgoState {
   int* seeds = nullptr;  // multi-seed BFS sources
   int nseeds_cap = 0;
   double* acc64 = nullptr;  // PPR adjoint scatter accumulator
-  double* pr_part = nullptr;  // row-word slices: one partial sum per long-row chunk
+  double* pr_part = nullptr;  // PageRank loop: every part's head and tail shares
   long long* push_list = nullptr;  // cooperative BFS: (start, tail offset) per listed long row
   void* scratch = nullptr;  // split partials (nslots * b * 8 bytes)
   cudaGraphExec_t exec[8] = {};
@@ -87,7 +89,7 @@ struct AlgoState {
   unsigned long long* stamps = nullptr;  // kStampCap + 1 iteration end times
   int launches_per_iter = 0;             // kernels of one loop iteration
   int fixed_launches = 2;                // kernels of a run outside its iterations
-  bool coop_run = false;                 // the last run was a cooperative BFS
+  bool coop_run = false;                 // the last run was a cooperative launch
   bool stats_pending = false;            // step times not yet read back
 
   // statistics of the last algorithm run
@@ -109,7 +111,7 @@ constexpr int kStepsPerGraph = 8;
 constexpr bool kCoopBfsDefault = true;
 constexpr int kCoopBlocksPerSM = 4;
 
-enum AlgoId { A_BFS = 0, A_SSSP = 1, A_PR = 2, A_CC = 3, A_PPR_F = 4, A_PPR_B = 5, A_PPR_BG = 6 };
+enum AlgoId { A_BFS = 0, A_CC = 1, A_PPR_B = 2 };
 
 template <int B>
 __device__ __forceinline__ typename Word<B>::T full_word() {
@@ -925,11 +927,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // or sees that another block gave up, sets bar_err and returns false: the
 // caller leaves the kernel, so every block ends within about one limit of
 // the first failure.
-__device__ __forceinline__ bool grid_barrier(Ctrl* c, unsigned long long limit_ns,
-                                             const unsigned long long* sum_src = nullptr, int nsum = 0,
-                                             int sum_stride = 1, unsigned long long* sum = nullptr) {
+template <typename T = unsigned long long>
+__device__ __forceinline__ bool grid_barrier(Ctrl* c, unsigned long long limit_ns, const T* sum_src = nullptr,
+                                             int nsum = 0, int sum_stride = 1, T* sum = nullptr) {
   __shared__ int ok;
-  __shared__ unsigned long long sh_sum;
+  __shared__ T sh_sum;
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned inc = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
@@ -949,7 +951,7 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* c, unsigned long long limit_n
     __threadfence();
     ok = res;
     // one read of the counters per block, shared with its threads
-    unsigned long long t = 0;
+    T t = 0;
     for (int q = 0; q < nsum; ++q) t += __ldcg(sum_src + (size_t)q * sum_stride);
     sh_sum = t;
   }
@@ -1137,8 +1139,7 @@ __global__ void k_level_to_dist(uint32_t* __restrict__ d, int n) {
 // adjoint on a symmetric P (row_scale) y = pv[i] + alpha * inv[i] * a with
 // a = sum of u[j].  Writes y (and y * inv[i], the next gathered operand, for
 // PageRank) and returns the |change| (or its square for the L2 norm).
-__device__ __forceinline__ double pr_row_update(long long i, double a, const float* __restrict__ x,
-                                                float* __restrict__ y, float* __restrict__ ys,
+__device__ __forceinline__ double pr_row_update(long long i, double a, const float* x, float* y, float* ys,
                                                 const float* __restrict__ inv, const float* __restrict__ pv,
                                                 double alpha, double add, double adds, int norm,
                                                 int row_scale) {
@@ -1150,291 +1151,109 @@ __device__ __forceinline__ double pr_row_update(long long i, double a, const flo
   return norm == 1 ? fabs(d) : d * d;
 }
 
-template <int B>
-__global__ void __launch_bounds__(kTPB) k_pr_step(GView v, float* __restrict__ pr, float* __restrict__ prs,
-                                                  const float* __restrict__ inv,
-                                                  const float* __restrict__ pv,
-                                                  Ctrl* __restrict__ ctrl, double* __restrict__ scratch) {
-  using L = Lay<B>;
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const int itn = ((volatile Ctrl*)ctrl)->iter;
-  const double alpha = ctrl->alpha, add = ctrl->add, adds = ctrl->add_scale;
-  const int norm = ctrl->norm, row_scale = ctrl->row_scale;
-  const int n = v.nrows;
-  const float* __restrict__ x = pr + (size_t)(itn & 1) * n;
-  float* __restrict__ y = pr + (size_t)((itn + 1) & 1) * n;
-  float* __restrict__ ys = prs + (size_t)((itn + 1) & 1) * n;
-  // gathered operand: x / deg (kept up to date by the previous iteration) or x
-  const float* __restrict__ xg = row_scale ? x : prs + (size_t)(itn & 1) * n;
+// The whole PageRank-type loop in one cooperative launch over the row lists
+// (gather.cuh), one block an SM.  Warps take parts in turn, sum their rows and
+// update those that began in the part; the next part's columns load
+// meanwhile.  Rows that cross parts leave their shares in `head` / `tail` and
+// are finished after a grid barrier, a thread per part they end in; a second
+// barrier closes the iteration, after which every block reads the same error
+// and takes the same decision.  The iterate is read with plain loads: the
+// barriers' fences make the other blocks' writes visible to them.
+//
+// Bound by the gathers of the iterate (a 32-byte sector of L2 each where L1
+// misses) and the instructions around them.  Per iteration: R-MAT 21 (62 M
+// set bits) 580 us as row-word walks in a loop graph, 226 now; R-MAT 18 140
+// and 38; 1,003 vertices 21 and 9 (two barriers); a mesh of 640,000 vertices
+// 32 and 28.  On the way, R-MAT 21: a block of 256 threads per part 316 (its
+// own barriers; 6 or 8 blocks an SM 360-410, they take L1 from the gathers),
+// a warp per part in a loop graph 282, ranges of adjacent parts per warp 440
+// (the ranges of low-degree rows finish last).
+__global__ void __launch_bounds__(kGatherTPB, 1)
+k_pr_loop(GatherList gl, float* pr, float* prs, const float* __restrict__ inv, const float* __restrict__ pv, Ctrl* ctrl,
+          double* head, double* tail, unsigned long long limit_ns) {
+  extern __shared__ __align__(16) unsigned char gather_sh[];
+  __shared__ double esh[kGatherWarps];
+  volatile Ctrl* vc = ctrl;
+  if (ctrl->done) return;
   const unsigned lane = threadIdx.x & 31;
-  double e = 0.0;
-  const long long nwarps = warps_total();
-  for (long long w = warp_global(); w * L::G < v.nitems; w += nwarps) {
-    const long long item = w * L::G + lane / L::W;
-    if (item < v.nitems) {
-      const int r = lane % L::W;
-      const gbo_item it = v.items[item];
-      double a0 = 0.0, a1 = 0.0;
-      fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r, [&](long long j) { return (double)xg[j]; },
-                          [](double& a, double b) { a += b; }, a0, a1);
-      if (it.slot >= 0) {
-        scratch[(size_t)it.slot * B + r] = a0;
-        if (L::RPL == 2) scratch[(size_t)it.slot * B + 32 + r] = a1;
-      } else {
-        const long long row0 = (long long)it.row * B + r;
-        if (row0 < n) e += pr_row_update(row0, a0, x, y, ys, inv, pv, alpha, add, adds, norm, row_scale);
-        if (L::RPL == 2 && row0 + 32 < n)
-          e += pr_row_update(row0 + 32, a1, x, y, ys, inv, pv, alpha, add, adds, norm, row_scale);
-      }
+  const int wib = (int)(threadIdx.x >> 5);
+  GatherShared& sh = reinterpret_cast<GatherShared*>(gather_sh)[wib];
+  const int i0 = (int)blockIdx.x + (int)gridDim.x * wib;  // neighbouring parts on different SMs
+  const int step = (int)gridDim.x * kGatherWarps;
+  const double alpha = ctrl->alpha, add = ctrl->add, adds = ctrl->add_scale, tol = ctrl->tol;
+  const double ref = ctrl->ref > 0.0 ? ctrl->ref : 1.0;  // ||w||_1 for the adjoint, else 1
+  const int norm = ctrl->norm, row_scale = ctrl->row_scale, n = gl.nrows, max_iter = ctrl->max_iter;
+  unsigned long long* stamps = ctrl->stamps;
+  for (int itn = ctrl->iter;;) {
+    const float* x0 = pr + (size_t)(itn & 1) * n;
+    float* y = pr + (size_t)((itn + 1) & 1) * n;
+    float* ys = prs + (size_t)((itn + 1) & 1) * n;
+    const float* xg = row_scale ? x0 : prs + (size_t)(itn & 1) * n;
+    double e = 0.0;
+    GatherPart p = {}, pn = {};
+    int c[kGatherItems];
+    if (i0 < gl.nparts) {
+      p = gl.part[i0];
+      gather_columns(gl, p, i0, lane, c);
     }
-  }
-  block_add_f64(e, &ctrl->err);
-}
-
-// The same iteration over the row-word slices of a b = 32 ROW graph: a warp
-// per block row, lane r sums row r's columns entry by entry (the head's
-// entry k of the 32 rows in one 256-byte load, two entries in flight), then
-// its tail.  Rows with tails longer than kRwsLongTail (hubs) are left to
-// k_pr_long_chunks / k_pr_long_rows, which spread them over many warps.
-// Every row's sum has a fixed order (fp64), whatever the grid.
-__device__ __forceinline__ double pr_word_sum(unsigned c, unsigned w, const float* __restrict__ xg) {
-  double a = 0.0;
-  const size_t base = (size_t)c * 32;
-  while (w) {
-    const int j = __clz(w);
-    a += (double)__ldg(xg + base + j);
-    w &= ~(0x80000000u >> j);
-  }
-  return a;
-}
-
-// Four entries at once: the gathered operand of one set column per entry
-// per round, four gathers in flight; the adds follow a fixed order (round,
-// then entry), so a row's sum depends on the graph only.
-__device__ __forceinline__ double pr_entries4(const uint2 (&e)[4], const float* __restrict__ xg) {
-  uint32_t m[4];
+    if (i0 + step < gl.nparts) pn = gl.part[i0 + step];
+    for (int i = i0; i < gl.nparts; i += step) {
+      float x[kGatherItems];
+      const int k = gather_count(gl, p, i);
 #pragma unroll
-  for (int u = 0; u < 4; ++u) m[u] = e[u].x != kRwsNone ? e[u].y : 0u;
-  double a = 0.0;
-  while (m[0] | m[1] | m[2] | m[3]) {
-    float g[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      g[u] = 0.f;
-      if (m[u]) {
-        const int j = __clz(m[u]);
-        m[u] &= ~(0x80000000u >> j);
-        g[u] = __ldg(xg + (size_t)e[u].x * 32 + j);
+      for (int u = 0; u < kGatherItems; ++u) x[u] = (int)lane + 32 * u < k ? xg[c[u]] : 0.f;
+      GatherPart pnn = {};
+      if (i + step < gl.nparts) gather_columns(gl, pn, i + step, lane, c);
+      if (i + 2 * step < gl.nparts) pnn = gl.part[i + 2 * step];
+      const double out = gather_reduce(gl, p, i, sh, lane, x);
+      for (int j = (int)lane; j < p.rows; j += 32) {
+        if (j == 0 && p.open) head[i] = sh.buf[0];
+        else e += pr_row_update(p.a0 + j, sh.buf[j], x0, y, ys, inv, pv, alpha, add, adds, norm, row_scale);
       }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) a += (double)g[u];
-  }
-  return a;
-}
-
-// The whole head (eight entries) at once: PageRank reads every entry of a
-// row, so the second half is not worth a round trip of its own.
-__device__ __forceinline__ double pr_entries8(const uint2 (&e)[8], const float* __restrict__ xg) {
-  uint32_t m[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) m[u] = e[u].x != kRwsNone ? e[u].y : 0u;
-  double a = 0.0;
-  while (m[0] | m[1] | m[2] | m[3] | m[4] | m[5] | m[6] | m[7]) {
-    float g[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      g[u] = 0.f;
-      if (m[u]) {
-        const int j = __clz(m[u]);
-        m[u] &= ~(0x80000000u >> j);
-        g[u] = __ldg(xg + (size_t)e[u].x * 32 + j);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) a += (double)g[u];
-  }
-  return a;
-}
-
-struct PrIter {  // the iterate's buffers and coefficients of iteration itn
-  const float* x;
-  float* y;
-  float* ys;
-  const float* xg;
-  double alpha, add, adds;
-  int norm, row_scale;
-};
-
-__device__ __forceinline__ PrIter pr_iter(float* pr, float* prs, const Ctrl* ctrl, int n) {
-  PrIter p;
-  const int itn = ((volatile Ctrl*)ctrl)->iter;
-  p.alpha = ctrl->alpha;
-  p.add = ctrl->add;
-  p.adds = ctrl->add_scale;
-  p.norm = ctrl->norm;
-  p.row_scale = ctrl->row_scale;
-  p.x = pr + (size_t)(itn & 1) * n;
-  p.y = pr + (size_t)((itn + 1) & 1) * n;
-  p.ys = prs + (size_t)((itn + 1) & 1) * n;
-  p.xg = p.row_scale ? p.x : prs + (size_t)(itn & 1) * n;
-  return p;
-}
-
-// Five blocks per SM (48 registers, a few spilled): the step is bound by the
-// latency of its gathers, and R-MAT 22 iterations took 1.05 ms at the 71
-// registers (3 blocks per SM) the compiler chose unbounded, 0.97 ms at 4
-// blocks and 0.90 ms at 5 to 8.
-__global__ void __launch_bounds__(kTPB, 5) k_pr_step_rws(GView v, float* __restrict__ pr, float* __restrict__ prs,
-                                                      const float* __restrict__ inv,
-                                                      const float* __restrict__ pv, Ctrl* __restrict__ ctrl) {
-  __shared__ double pr_tail_sh[kTPB / 32][32];
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const int n = v.nrows;
-  const PrIter P = pr_iter(pr, prs, ctrl, n);
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned kFull = 0xffffffffu;
-  double e = 0.0;
-  const long long nwarps = warps_total();
-  for (long long R = warp_global(); R < v.nbr; R += nwarps) {
-    const long long row = R * 32 + lane;
-    const uint2* __restrict__ hp = v.rws_head + (size_t)R * (kRwsHead * 32) + lane;
-    // the head's eight entries and the tail offsets in one round of loads
-    static_assert(kRwsHead == 8, "pr_entries8 takes the whole head");
-    uint2 h8[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) h8[u] = hp[(size_t)u * 32];
-    const long long tb = v.rws_tail_ptr[row], te = v.rws_tail_ptr[row + 1];
-    double a = pr_entries8(h8, P.xg);
-    const bool long_row = te - tb > kRwsLongTail;  // the chunk kernels own a long row
-    // The block row's short tails as one list, 32 entries per round over the
-    // warp's lanes (a lane per row would wait for the block row's longest
-    // tail): lane q of a round finds its entry's row r by a binary search
-    // over the tails' inclusive sums, and a segmented scan across the lanes
-    // adds each row's entries of the round, in lane order, into tsum[r].
-    const int len = long_row ? 0 : (int)(te - tb);
-    const int incl = warp_incl_sum(len, lane);
-    const int total = __shfl_sync(kFull, incl, 31);
-    double* tsum = pr_tail_sh[threadIdx.x >> 5];
-    tsum[lane] = 0.0;
-    __syncwarp();
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int q = p0 + (int)lane;
-      int r = 0;
-#pragma unroll
-      for (int st = 16; st > 0; st >>= 1)
-        if (__shfl_sync(kFull, incl, r + st - 1) <= q) r += st;
-      const int rin = __shfl_sync(kFull, incl, r);
-      const int rlen = __shfl_sync(kFull, len, r);
-      const long long rtb = __shfl_sync(kFull, tb, r);
-      double val = 0.0;
-      if (q < total) {
-        const uint2 t = v.rws_tail[rtb + (q - (rin - rlen))];
-        for (uint32_t m = t.y; m;) {
-          const int j = __clz(m);
-          m &= ~(0x80000000u >> j);
-          val += (double)__ldg(P.xg + (size_t)t.x * 32 + j);
-        }
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(kFull, val, o);
-        const int ry = __shfl_up_sync(kFull, r, o);
-        if ((int)lane >= o && ry == r) val += y;
-      }
-      const int rn = __shfl_down_sync(kFull, r, 1);
-      if (q < total && (lane == 31 || q + 1 == total || rn != r)) tsum[r] += val;
+      if (lane == 0) tail[i] = out;
       __syncwarp();
+      p = pn;
+      pn = pnn;
     }
-    a += tsum[lane];
-    if (row < n && !long_row)
-      e += pr_row_update(row, a, P.x, P.y, P.ys, inv, pv, P.alpha, P.add, P.adds, P.norm, P.row_scale);
-  }
-  block_add_f64(e, &ctrl->err);
-}
-
-// Long rows, part 1: a warp per chunk of a long row's tail sums its entries
-// (lanes strided, partial sums combined by a fixed shuffle tree); the first
-// chunk of a row also sums the row's head.  One fp64 partial per chunk.
-__global__ void __launch_bounds__(kTPB) k_pr_long_chunks(GView v, float* __restrict__ pr,
-                                                         float* __restrict__ prs, Ctrl* __restrict__ ctrl,
-                                                         double* __restrict__ part) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const PrIter P = pr_iter(pr, prs, ctrl, v.nrows);
-  const unsigned lane = threadIdx.x & 31;
-  const long long nwarps = warps_total();
-  for (long long q = warp_global(); q < v.rws_nchunk; q += nwarps) {
-    const long long row = v.rws_chunk_row[q];
-    const long long b = v.rws_chunk_beg[q], e = v.rws_chunk_end[q];
-    double a = 0.0;
-    if (b == v.rws_tail_ptr[row] && lane < kRwsHead) {
-      const uint2 h = v.rws_head[((size_t)(row >> 5) * kRwsHead + lane) * 32 + (row & 31)];
-      a += pr_word_sum(h.x, h.y, P.xg);  // a long row fills its head
-    }
-    for (long long p = b + lane; p < e; p += 128) {
-      uint2 t[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) t[u] = p + 32 * u < e ? v.rws_tail[p + 32 * u] : make_uint2(kRwsNone, 0u);
-      a += pr_entries4(t, P.xg);
+    if (!grid_barrier(ctrl, limit_ns)) return;
+    for (int b = (int)(blockIdx.x * blockDim.x) + wib * 32; b < gl.nparts; b += (int)(gridDim.x * blockDim.x)) {
+      const int i = b + (int)lane;
+      GatherPart q = {};
+      if (i < gl.nparts) q = gl.part[i];
+      const bool want = q.open && q.rows > 0;
+      const double a = gather_open_sum(gl, q, i, want, head, tail);
+      if (want) e += pr_row_update(q.a0, a, x0, y, ys, inv, pv, alpha, add, adds, norm, row_scale);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) part[q] = a;
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (lane == 0) esh[wib] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 1; q < kGatherWarps; ++q) e += esh[q];
+      if (e != 0.0) atomicAdd(&ctrl->err_part[itn % 3][blockIdx.x & 7][0], e);
+    }
+    double err = 0.0;
+    if (!grid_barrier(ctrl, limit_ns, &ctrl->err_part[itn % 3][0][0], 8, 16, &err)) return;
+    const int it = itn + 1;
+    const double m = norm == 2 ? sqrt(err) : err;
+    const bool stop = it >= max_iter || (tol >= 0.0 && m <= tol * ref);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      for (int q = 0; q < 8; ++q) ctrl->err_part[(itn + 2) % 3][q][0] = 0.0;
+      vc->iter = it;
+      vc->last_err = err;
+      if (stop) vc->done = 1;
+      if (stamps && it <= kStampCap) stamps[it] = global_ns();
+      __threadfence();
+    }
+    if (stop) return;
+    itn = it;
   }
-}
-
-// Long rows, part 2: a thread per long row adds its chunks' partials in
-// chunk order and updates the row.
-__global__ void k_pr_long_rows(GView v, float* __restrict__ pr, float* __restrict__ prs,
-                               const float* __restrict__ inv, const float* __restrict__ pv,
-                               Ctrl* __restrict__ ctrl, const double* __restrict__ part) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const PrIter P = pr_iter(pr, prs, ctrl, v.nrows);
-  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double e = 0.0;
-  if (q < v.rws_nlong) {
-    const long long row = v.rws_long_row[q];
-    double a = 0.0;
-    for (long long c = v.rws_long_chunk0[q]; c < v.rws_long_chunk0[q + 1]; ++c) a += part[c];
-    if (row < v.nrows)
-      e = pr_row_update(row, a, P.x, P.y, P.ys, inv, pv, P.alpha, P.add, P.adds, P.norm, P.row_scale);
-  }
-  block_add_f64(e, &ctrl->err);
-}
-
-template <int B>
-__global__ void k_pr_finish(GView v, float* __restrict__ pr, float* __restrict__ prs,
-                            const float* __restrict__ inv, const float* __restrict__ pv,
-                            Ctrl* __restrict__ ctrl, const double* __restrict__ scratch) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const int itn = ((volatile Ctrl*)ctrl)->iter;
-  const double alpha = ctrl->alpha, add = ctrl->add, adds = ctrl->add_scale;
-  const int norm = ctrl->norm, row_scale = ctrl->row_scale;
-  const int n = v.nrows;
-  const float* __restrict__ x = pr + (size_t)(itn & 1) * n;
-  float* __restrict__ y = pr + (size_t)((itn + 1) & 1) * n;
-  float* __restrict__ ys = prs + (size_t)((itn + 1) & 1) * n;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double e = 0.0;
-  if (gid < (long long)v.nsplit * B) {
-    const gbo_split sp = v.splits[gid / B];
-    const int r = (int)(gid % B);
-    double a = 0.0;
-    for (int q = 0; q < sp.nslots; ++q) a += scratch[(size_t)(sp.slot0 + q) * B + r];
-    const long long row = (long long)sp.row * B + r;
-    if (row < n) e += pr_row_update(row, a, x, y, ys, inv, pv, alpha, add, adds, norm, row_scale);
-  }
-  block_add_f64(e, &ctrl->err);
-  close_iteration(ctrl, [](volatile Ctrl* c, int it) {
-    const double m = c->norm == 2 ? sqrt(c->err) : c->err;
-    const double ref = c->ref > 0.0 ? c->ref : 1.0;  // ||w||_1 for the adjoint, else 1
-    return it >= c->max_iter || (c->tol >= 0.f && m <= (double)c->tol * ref);
-  });
 }
 
 __global__ void k_pr_init(float* pr, float* prs, const float* inv, const float* pv, int n,
                           float init_const, float init_scale, Ctrl* ctrl, int max_iter, float tol,
-                          float alpha, float add, float add_scale, int norm, int row_scale) {
+                          float alpha, float add, float add_scale, int norm, int row_scale,
+                          unsigned long long* stamps = nullptr, int cap_iters = 0) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long k = i; k < n; k += stride) {
@@ -1450,10 +1269,16 @@ __global__ void k_pr_init(float* pr, float* prs, const float* inv, const float* 
     ctrl->iter = 0;
     ctrl->done = max_iter <= 0 ? 1 : 0;
     ctrl->ticket = 0;
-    ctrl->max_iter = max_iter;
+    ctrl->max_iter = cap_iters > 0 && cap_iters < max_iter ? cap_iters : max_iter;
+    if (stamps) {  // a cooperative loop's start
+      ctrl->cond = 0ull;
+      ctrl->stamps = stamps;
+      stamps[0] = global_ns();
+    }
     ctrl->count = 0;
     ctrl->err = 0;
     ctrl->last_err = 0;
+    ctrl->bar_arrive = 0u;
     ctrl->bar_err = 0u;
     ctrl->tol = tol;
     ctrl->alpha = alpha;
@@ -1464,6 +1289,7 @@ __global__ void k_pr_init(float* pr, float* prs, const float* inv, const float* 
     ctrl->ref = 0.0;
     ctrl->row_scale = row_scale;
   }
+  if (i < 3 * 8) ctrl->err_part[i / 8][i % 8][0] = 0.0;
 }
 
 // ===================================================== PPR adjoint step
@@ -1821,13 +1647,6 @@ int ensure_pr_vectors(gbo_graph* g, AlgoState* a) {
   return GBO_OK;
 }
 
-int ensure_pr_part(gbo_graph* g, AlgoState* a) {
-  if (a->pr_part || g->rws_nchunk <= 0) return GBO_OK;
-  GBO_CUDA_TRY(cudaMalloc(&a->pr_part, sizeof(double) * (size_t)g->rws_nchunk));
-  g->device_bytes += 8LL * g->rws_nchunk;
-  return GBO_OK;
-}
-
 int ensure_vec_i32(gbo_graph* g, int** p) {
   if (!*p) {
     GBO_CUDA_TRY(cudaMalloc(p, sizeof(int) * (size_t)(g->nrows > 0 ? g->nrows : 1)));
@@ -1902,7 +1721,7 @@ int finish_loop(AlgoState* a, cudaStream_t s, int max_iter, int cap_iters, int* 
   if (!iters && cap_iters == 0 && !must_wait) return GBO_OK;
   GBO_CUDA_TRY(cudaMemcpyAsync(a->h_ctrl, a->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
   GBO_CUDA_TRY(cudaStreamSynchronize(s));
-  if (coop && a->h_ctrl->bar_err) return fail(GBO_ERR_TIMEOUT, "cooperative BFS: a grid barrier gave up");
+  if (coop && a->h_ctrl->bar_err) return fail(GBO_ERR_TIMEOUT, "cooperative loop: a grid barrier gave up");
   if (!a->h_ctrl->done) return fail(GBO_ERR_TIMEOUT, "iteration loop did not terminate");
   if (cap_iters > 0 && cap_iters < max_iter && a->h_ctrl->iter >= cap_iters)
     return fail(GBO_ERR_TIMEOUT, "iteration loop cut off by the injected cap");
@@ -1974,8 +1793,8 @@ int collect_stats(AlgoState* a) {
   a->stats_pending = false;
   GBO_CUDA_TRY(cudaDeviceSynchronize());
   GBO_CUDA_TRY(cudaMemcpy(a->h_ctrl, a->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
-  // a stream-ordered cooperative BFS whose grid barrier gave up reports it here
-  if (a->coop_run && a->h_ctrl->bar_err) return fail(GBO_ERR_TIMEOUT, "cooperative BFS: a grid barrier gave up");
+  // a stream-ordered cooperative loop whose grid barrier gave up reports it here
+  if (a->coop_run && a->h_ctrl->bar_err) return fail(GBO_ERR_TIMEOUT, "cooperative loop: a grid barrier gave up");
   const int it = a->h_ctrl->iter;
   const int nst = std::min(it, kStampCap);
   std::vector<unsigned long long> t((size_t)nst + 1);
@@ -2098,54 +1917,51 @@ int sssp_impl(gbo_graph* g, int src, uint32_t* d_dist, int* h_iters, cudaStream_
   return GBO_OK;
 }
 
+// The PageRank-type loop (pv: the personalization or the adjoint's w, or NULL)
+// after k_pr_init: one cooperative launch, a block an SM.
+int run_pr_loop(gbo_graph* g, AlgoState* a, const float* pv, int max_iter, int cap_iters, int* iters, cudaStream_t s) {
+  GatherList gl = gather_of(g);
+  int per_sm = 0;
+  const size_t smem = sizeof(GatherShared) * kGatherWarps;
+  GBO_CUDA_TRY(cudaFuncSetAttribute(k_pr_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_loop, kGatherTPB, smem));
+  if (per_sm < 1) return fail(GBO_ERR_UNSUPPORTED, "PageRank loop kernel does not fit an SM");
+  // every SM from a few parts a block on (a barrier over few blocks is cheaper)
+  const int grid = std::max(1, std::min((gl.nparts + 3) / 4, num_sms()));
+  const size_t np = (size_t)std::max(gl.nparts, 1);
+  if (!a->pr_part) {
+    GBO_CUDA_TRY(cudaMalloc(&a->pr_part, sizeof(double) * 2 * np));
+    g->device_bytes += 16LL * (long long)np;
+  }
+  float *pr = a->pr, *prs = a->prs;
+  const float* inv = g->invdeg;
+  Ctrl* ctrl = a->ctrl;
+  double *head = a->pr_part, *tail = a->pr_part + np;
+  unsigned long long limit_ns = kBarrierLimitNs;
+  void* args[] = {&gl, &pr, &prs, &inv, &pv, &ctrl, &head, &tail, &limit_ns};
+  GBO_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pr_loop, dim3((unsigned)grid), dim3(kGatherTPB), args, smem, s));
+  a->fixed_launches = 2;  // init and the loop
+  a->coop_run = true;
+  a->launches_per_iter = 0;
+  return finish_loop(a, s, max_iter, cap_iters, iters, true);
+}
+
 // Shared by PageRank (v = NULL) and the PPR forward pass.
-template <int B>
 int pr_impl(gbo_graph* g, const float* d_v, float alpha, int max_iter, float tol, float* d_p,
             int* h_iters, int norm, float init_const, float init_scale, float add, float add_scale,
-            int id, cudaStream_t s) {
+            cudaStream_t s) {
   AlgoState* a = nullptr;
   GBO_TRY(get_state(g, &a));
   GBO_TRY(ensure_pr_vectors(g, a));
-  GView v = view_of(g);
+  GBO_TRY(build_gather(g, s));
+  const int cap_iters = injected_cap_iters();
   float* pr = a->pr;
-  float* prs = a->prs;
-  const float* inv = g->invdeg;
-  Ctrl* ctrl = a->ctrl;
-  double* scratch = (double*)a->scratch;
-  // b = 32 ROW graphs iterate over their row-word slices (no split rows)
-  if (B == 32 && g->layout == GBO_LAYOUT_ROW) GBO_TRY(build_rws(g, s));
-  const bool rws = B == 32 && g->layout == GBO_LAYOUT_ROW && g->rws_head != nullptr;
-  if (rws) v = view_of(g);
-  GView vfin = v;
-  if (rws) vfin.nsplit = 0;
-  if (rws) GBO_TRY(ensure_pr_part(g, a));
-  const unsigned gi = rws ? grid_persistent(k_pr_step_rws, g->nbr)
-                          : grid_items_persistent(k_pr_step<B>, g->nitems, B);
-  const unsigned gc = rws ? grid_persistent(k_pr_long_chunks, std::max<long long>(g->rws_nchunk, 1)) : 1;
-  const unsigned gs = blocks_for((long long)vfin.nsplit * B, kTPB);
-  GBO_TRY(get_exec(a, id, d_v, [&](cudaStream_t cs, int k, int* nl) -> int {
-    if (g->nitems > 0) {
-      if (rws) {
-        k_pr_step_rws<<<gi, kTPB, 0, cs>>>(v, pr, prs, inv, d_v, ctrl);
-        if (g->rws_nchunk > 0) {
-          k_pr_long_chunks<<<gc, kTPB, 0, cs>>>(v, pr, prs, ctrl, a->pr_part);
-          k_pr_long_rows<<<blocks_for(g->rws_nlong, kTPB), kTPB, 0, cs>>>(v, pr, prs, inv, d_v, ctrl, a->pr_part);
-          *nl += 2;
-        }
-      } else {
-        k_pr_step<B><<<gi, kTPB, 0, cs>>>(v, pr, prs, inv, d_v, ctrl, scratch);
-      }
-    }
-    k_pr_finish<B><<<gs, kTPB, 0, cs>>>(vfin, pr, prs, inv, d_v, ctrl, scratch);
-    *nl += (g->nitems > 0) + 1;
-    GBO_CUDA_TRY(cudaGetLastError());
-    return GBO_OK;
-  }));
-  k_pr_init<<<grid_vertex(g->nrows), kTPB, 0, s>>>(pr, prs, inv, d_v, g->nrows, init_const, init_scale,
-                                                  ctrl, max_iter, tol, alpha, add, add_scale, norm, 0);
+  k_pr_init<<<grid_vertex(g->nrows), kTPB, 0, s>>>(pr, a->prs, g->invdeg, d_v, g->nrows, init_const, init_scale,
+                                                  a->ctrl, max_iter, tol, alpha, add, add_scale, norm, 0, a->stamps,
+                                                  cap_iters);
   GBO_CUDA_TRY(cudaGetLastError());
   int iters = 0;
-  if (max_iter > 0) GBO_TRY(run_until_done(a, id, s, max_iter, &iters));
+  if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_v, max_iter, cap_iters, &iters, s));
   if (g->nrows > 0)
     GBO_CUDA_TRY(cudaMemcpyAsync(d_p, pr + (size_t)(iters & 1) * g->nrows,
                                  sizeof(float) * (size_t)g->nrows, cudaMemcpyDeviceToDevice, s));
@@ -2165,45 +1981,16 @@ int ppr_backward_impl(gbo_graph* g, const float* d_w, float alpha, float tol, in
   if (g->symmetric) {
     // P^T = P: u' = w + alpha * D^-1 P u is a gather over P's rows (the
     // PageRank step with the scale on rows), no scatter atomics
+    GBO_TRY(build_gather(g, s));
+    const int cap_iters = injected_cap_iters();
     float* pr = a->pr;
-    float* prs = a->prs;
-    const float* inv = g->invdeg;
     Ctrl* ctrl = a->ctrl;
-    double* scratch = (double*)a->scratch;
-    if (B == 32 && g->layout == GBO_LAYOUT_ROW) GBO_TRY(build_rws(g, s));
-    const bool rws = B == 32 && g->layout == GBO_LAYOUT_ROW && g->rws_head != nullptr;
-    GView v = view_of(g);
-    GView vfin = v;
-    if (rws) vfin.nsplit = 0;
-    if (rws) GBO_TRY(ensure_pr_part(g, a));
-    const unsigned gi = rws ? grid_persistent(k_pr_step_rws, g->nbr)
-                            : grid_items_persistent(k_pr_step<B>, g->nitems, B);
-    const unsigned gc = rws ? grid_persistent(k_pr_long_chunks, std::max<long long>(g->rws_nchunk, 1)) : 1;
-    const unsigned gs = blocks_for((long long)vfin.nsplit * B, kTPB);
-    GBO_TRY(get_exec(a, A_PPR_BG, d_w, [&](cudaStream_t cs, int k, int* nl) -> int {
-      if (g->nitems > 0) {
-        if (rws) {
-          k_pr_step_rws<<<gi, kTPB, 0, cs>>>(v, pr, prs, inv, d_w, ctrl);
-          if (g->rws_nchunk > 0) {
-            k_pr_long_chunks<<<gc, kTPB, 0, cs>>>(v, pr, prs, ctrl, a->pr_part);
-            k_pr_long_rows<<<blocks_for(g->rws_nlong, kTPB), kTPB, 0, cs>>>(v, pr, prs, inv, d_w, ctrl, a->pr_part);
-            *nl += 2;
-          }
-        } else {
-          k_pr_step<B><<<gi, kTPB, 0, cs>>>(v, pr, prs, inv, d_w, ctrl, scratch);
-        }
-      }
-      k_pr_finish<B><<<gs, kTPB, 0, cs>>>(vfin, pr, prs, inv, d_w, ctrl, scratch);
-      *nl += (g->nitems > 0) + 1;
-      GBO_CUDA_TRY(cudaGetLastError());
-      return GBO_OK;
-    }));
     // u0 = w; y = w + alpha * inv * (P u)
     k_pr_init<<<gv, kTPB, 0, s>>>(pr, nullptr, nullptr, d_w, n, 0.f, 1.f, ctrl, max_iter, tol, alpha,
-                                  0.f, 1.f, 1, 1);
+                                  0.f, 1.f, 1, 1, a->stamps, cap_iters);
     k_l1_ref<<<gv, kTPB, 0, s>>>(d_w, n, ctrl);
     GBO_CUDA_TRY(cudaGetLastError());
-    if (max_iter > 0) GBO_TRY(run_until_done(a, A_PPR_BG, s, max_iter, &iters));
+    if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_w, max_iter, cap_iters, &iters, s));
     if (n > 0) k_scale_copy<<<gv, kTPB, 0, s>>>(pr + (size_t)(iters & 1) * n, d_grad, n, 1.f - alpha);
     GBO_CUDA_TRY(cudaGetLastError());
     if (h_iters) *h_iters = iters;
@@ -2472,8 +2259,8 @@ extern "C" int gbo_pagerank(const gbo_graph* gc, float alpha, int max_iter, floa
   if (max_iter < 0) return fail(GBO_ERR_INVALID, "max_iter < 0");
   const float n = (float)(g->nrows > 0 ? g->nrows : 1);
   int st = GBO_OK;
-  ALGO_DISPATCH_B(g->b, st = pr_impl<B>(g, nullptr, alpha, max_iter, tol, d_p, h_iters, 2, 1.0f / n,
-                                         0.f, (1.0f - alpha) / n, 0.f, A_PR, as_stream(stream)));
+  st = pr_impl(g, nullptr, alpha, max_iter, tol, d_p, h_iters, 2, 1.0f / n, 0.f, (1.0f - alpha) / n, 0.f,
+               as_stream(stream));
   return st;
 }
 
@@ -2497,8 +2284,8 @@ extern "C" int gbo_ppr_forward(const gbo_graph* gc, const float* d_v, float alph
   if (max_iter < 0) return fail(GBO_ERR_INVALID, "max_iter < 0");
   int st = GBO_OK;
   // p0 = (1-alpha) v;  p' = alpha P D^-1 p + (1-alpha) v
-  ALGO_DISPATCH_B(g->b, st = pr_impl<B>(g, d_v, alpha, max_iter, tol, d_p, h_iters, 1, 0.f,
-                                         1.f - alpha, 0.f, 1.f - alpha, A_PPR_F, as_stream(stream)));
+  st = pr_impl(g, d_v, alpha, max_iter, tol, d_p, h_iters, 1, 0.f, 1.f - alpha, 0.f, 1.f - alpha,
+               as_stream(stream));
   return st;
 }
 

@@ -126,6 +126,7 @@ void destroy(gbo_graph* g) {
   cudaFree(g->ws);
   free_algo_state(g);
   free_ms_state(g);
+  free_gather(g);
   delete g;
 }
 

@@ -55,6 +55,13 @@ struct gbo_graph {
   long long* rws_chunk_beg = nullptr;  // tail entries [beg, end) of every chunk
   long long* rws_chunk_end = nullptr;
   unsigned* rws_longbits = nullptr;    // nbr words: bit 31 - r set when row 32R + r is long
+  // the set columns of every row and the parts of a balanced walk over them
+  // (gather.cuh), built on first PageRank-type use
+  long long* gl_ptr = nullptr;  // nrows + 1
+  int* gl_col = nullptr;
+  void* gl_part = nullptr;      // gl_nparts parts (GatherPart)
+  long long gl_nnz = 0;
+  int gl_nparts = -1;           // -1: not built
   int last_run_ms = 0;     // 1: the last traversal was a multi-source BFS
   bool tc_mma = false;     // GBO_FLAG_TC_MMA: dense 32x32 mask tiles on the 1-bit MMA
   bool owns_outdeg = true;
@@ -135,6 +142,7 @@ void launch_invdeg(const int* d_deg, int n, float* d_inv, cudaStream_t stream);
 // Release the algorithm state of g (called by gbo_graph_free).
 void free_algo_state(gbo_graph* g);
 void free_ms_state(gbo_graph* g);
+void free_gather(gbo_graph* g);
 // Statistics of the last multi-source BFS (per-level times of its step kernel).
 int ms_last_run(const gbo_graph* g, gbo_run_stats* stats);
 
