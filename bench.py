@@ -1055,7 +1055,7 @@ def suite_config2(args, which):
         ms = _timed(gbo, lambda: gbo.check(gbo.lib().gbo_cc(g.h, buf.ptr, C.byref(it), None)),
                     args.steps, args.warmup)
         und = csr.nnz // 2
-        cfg["workload"] = f"connected components (FastSV, min label), R-MAT scale {args.scale}"
+        cfg["workload"] = f"connected components (min label), R-MAT scale {args.scale}"
         extra = {"iterations": it.value, "undirected_edges": und, "dtype": "i32"}
         if bs is not None:
             got = buf.to_numpy(np.int32, n)

@@ -2,13 +2,13 @@
 //
 // The reference loops (algorithm/bfs.cu:508-564, sssp.cu:420-470,
 // pr.cu:449-513, cc.cu:223-287) launch 5-9 kernels per iteration and copy a
-// convergence scalar to the host every iteration.  Here each iteration is one
-// fused step kernel plus a small kernel that finishes split block rows; the
-// last block of that kernel (atomic ticket) decides termination on the
-// device.  One iteration is captured once as the body of a conditional WHILE
-// node of a CUDA graph, and the deciding block clears the node's condition
-// when the loop stops: a whole traversal or solve is one graph launch with
-// no host round trip and no idle iterations.
+// convergence scalar to the host every iteration.  Here termination is decided
+// on the device: BFS on 32x32 tiles and the PageRank-type loops are one
+// cooperative launch whose blocks meet at grid barriers; the other widths' BFS
+// and the scattered adjoint are a CUDA graph with a conditional WHILE node
+// whose body is one iteration (the last block of its closing kernel, by an
+// atomic ticket, clears the condition); connected components are a fixed
+// sequence of kernels.  No host round trip and no idle iterations.
 #include <string.h>
 
 #include <algorithm>
@@ -70,13 +70,11 @@ struct AlgoState {
   void* live = nullptr;    // nbr words: bit set where the row of P has an entry
   int* level = nullptr;    // n
   uint32_t* dist = nullptr;
-  // PR / PPR / CC vectors
+  // PR / PPR vectors
   float* pr = nullptr;     // 2 * n
   float* prs = nullptr;    // 2 * n: the iterate scaled by D^-1 (PageRank gathers it)
   const float* ppr_v = nullptr;
-  int* f = nullptr;
-  int* gf = nullptr;
-  int* mngf = nullptr;
+  void* cc = nullptr;       // connected components: CcState and the list of long rows
   int* seeds = nullptr;  // multi-seed BFS sources
   int nseeds_cap = 0;
   double* acc64 = nullptr;  // PPR adjoint scatter accumulator
@@ -111,7 +109,7 @@ constexpr int kStepsPerGraph = 8;
 constexpr bool kCoopBfsDefault = true;
 constexpr int kCoopBlocksPerSM = 4;
 
-enum AlgoId { A_BFS = 0, A_CC = 1, A_PPR_B = 2 };
+enum AlgoId { A_BFS = 0, A_PPR_B = 1 };
 
 template <int B>
 __device__ __forceinline__ typename Word<B>::T full_word() {
@@ -1372,166 +1370,213 @@ __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ 
 }
 
 // ================================================================== CC
-// FastSV (Zhang, Azad, Hu 2020): min-neighbour grandparent, stochastic and
-// aggressive hooking, shortcutting, until the grandparents stop changing.
-template <int B>
-__global__ void __launch_bounds__(kTPB) k_cc_mngf(GView v, const int* __restrict__ gf,
-                                                  int* __restrict__ mngf, Ctrl* __restrict__ ctrl,
-                                                  int* __restrict__ scratch) {
-  using WT = typename Word<B>::T;
-  using L = Lay<B>;
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const unsigned lane = threadIdx.x & 31;
-  const long long nwarps = warps_total();
-  for (long long w = warp_global(); w * L::G < v.nitems; w += nwarps) {
-    const long long item = w * L::G + lane / L::W;
-    if (item >= v.nitems) continue;
-    const int r = lane % L::W;
-    const gbo_item it = v.items[item];
-    int a0 = kINF, a1 = kINF;
-    fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r, [&](long long j) { return gf[j]; },
-                        [](int& a, int b) { a = min(a, b); }, a0, a1);
-    if (it.slot >= 0) {
-      scratch[(size_t)it.slot * B + r] = a0;
-      if (L::RPL == 2) scratch[(size_t)it.slot * B + 32 + r] = a1;
-      continue;
-    }
-    const long long row0 = (long long)it.row * B + r;
-    if (row0 < v.nrows && a0 < mngf[row0]) mngf[row0] = a0;
-    if (L::RPL == 2 && row0 + 32 < v.nrows && a1 < mngf[row0 + 32]) mngf[row0 + 32] = a1;
-  }
-}
+// Afforest (Sutton, Ben-Nun, Barak, "Optimizing Parallel Graph Connectivity
+// Computation via Subgraph Sampling", IPDPS 2018) over the row lists: a
+// forest in the caller's label array whose links always go from a higher to a
+// lower vertex, so a component's root is its smallest vertex.  Two edges per
+// vertex link most of a graph's largest component; a sample of the labels
+// names it, and only the vertices outside it go through all their edges (an
+// edge between the two sides is seen from the outside one: P is symmetric).
+//
+// Bound by the random accesses to the labels (a handful per vertex).  The
+// FastSV loop this replaces gathered a label per set bit in each of its four
+// to six iterations and ran five kernels in each.  Before / now (us): R-MAT 20
+// with shuffled labels 1,230 / 182, R-MAT 21 1,669 / 175, a mesh of 10^6
+// vertices 501 / 111, random graphs of 10^6 vertices and average degree 1 and
+// 3 440 / 120 and 571 / 221, 1,003 vertices 90 / 54.
+constexpr int kCcSamples = 256;
+constexpr int kCcChunk = 2048;  // set bits of a long row that one warp takes
+constexpr int kCcShort = 8;     // rows up to this many set bits are one lane's
 
-// The same minimum over the row-word slices of a 32x32 ROW graph: a warp per
-// block row, lane r over row r's entries (the whole head in one round, then
-// tails of up to kRwsLongTail entries four at a time), the grandparent of
-// every column of each entry gathered; longer tails are k_cc_mngf_chunks'.
-__device__ __forceinline__ int cc_min_entries(const uint2* e, int ne, const int* __restrict__ gf, int a) {
-  for (int u = 0; u < ne; ++u) {
-    if (e[u].x == kRwsNone) continue;
-    for (uint32_t m = e[u].y; m;) {
-      const int j = __clz(m);
-      m &= ~(0x80000000u >> j);
-      a = min(a, __ldg(gf + (size_t)e[u].x * 32 + j));
+// cc_root halves the path it walks (every vertex passed moves to its
+// grandparent, as ECL-CC's intermediate pointer jumping: Jaiganesh and
+// Burtscher, HPDC 2018): a mesh starts as paths of a thousand vertices.  A
+// stored parent is always an ancestor and only roots are hooked, by CAS, so
+// these plain stores never undo a link.  Labels are read through L1, where
+// they may be out of date: an old label is an ancestor too, and a link whose
+// root has been hooked meanwhile learns its new parent from the CAS.  (Read
+// from L2, the last pass of the random graph of average degree 3 took 1,175
+// us instead of 420, before k_cc_hook's passes left little to it.)
+__device__ __forceinline__ int cc_root(int* comp, int v) {
+  int cur = __ldca(comp + v);
+  if (cur != v) {
+    int prev = v;
+    for (int next = __ldca(comp + cur); next != cur; next = __ldca(comp + cur)) {
+      comp[prev] = next;
+      prev = cur;
+      cur = next;
     }
   }
-  return a;
+  return cur;
 }
 
-__global__ void __launch_bounds__(kTPB) k_cc_mngf_rws(GView v, const int* __restrict__ gf, int* __restrict__ mngf,
-                                                      Ctrl* __restrict__ ctrl) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const unsigned lane = threadIdx.x & 31;
-  const long long nwarps = warps_total();
-  for (long long R = warp_global(); R < v.nbr; R += nwarps) {
-    const long long row = R * 32 + lane;
-    const uint2* __restrict__ hp = v.rws_head + (size_t)R * (kRwsHead * 32) + lane;
-    uint2 h8[kRwsHead];
-#pragma unroll
-    for (int u = 0; u < kRwsHead; ++u) h8[u] = hp[(size_t)u * 32];
-    const long long tb = v.rws_tail_ptr[row], te = v.rws_tail_ptr[row + 1];
-    int a = cc_min_entries(h8, kRwsHead, gf, kINF);
-    if (te - tb <= kRwsLongTail) {
-      for (long long p = tb; p < te; p += 4) {
-        uint2 e[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) e[u] = p + u < te ? v.rws_tail[p + u] : make_uint2(kRwsNone, 0u);
-        a = cc_min_entries(e, 4, gf, a);
-      }
-    }
-    if (row < v.nrows && a < mngf[row]) mngf[row] = a;
+__device__ __forceinline__ void cc_link(int* comp, int u, int v) {
+  int a = cc_root(comp, u), b = cc_root(comp, v);
+  while (a != b) {  // every turn ends or replaces the higher vertex by a lower one
+    const int hi = max(a, b), lo = min(a, b);
+    const int old = atomicCAS(comp + hi, hi, lo);
+    if (old == hi) return;
+    a = old;
+    b = lo;
   }
 }
 
-// Long tails: a warp per chunk, the chunk's minimum folded into its row with
-// atomicMin (after k_cc_mngf_rws wrote the row's head and short part).
-__global__ void __launch_bounds__(kTPB) k_cc_mngf_chunks(GView v, const int* __restrict__ gf,
-                                                         int* __restrict__ mngf, Ctrl* __restrict__ ctrl) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const unsigned lane = threadIdx.x & 31;
-  const long long nwarps = warps_total();
-  for (long long q = warp_global(); q < v.rws_nchunk; q += nwarps) {
-    const long long e0 = v.rws_chunk_end[q];
-    int a = kINF;
-    for (long long p = v.rws_chunk_beg[q] + lane; p < e0; p += 32) {
-      const uint2 e = v.rws_tail[p];
-      a = cc_min_entries(&e, 1, gf, a);
-    }
-    a = __reduce_min_sync(0xffffffffu, a);
-    const long long row = v.rws_chunk_row[q];
-    if (lane == 0 && row < v.nrows && a < mngf[row]) atomicMin(mngf + row, a);
-  }
-}
+// State of a run beside the labels: the sampled largest component, the lists
+// of long rows outside it (rows << 40 | chunks, as the BFS push list) of the
+// two passes, and whether the first pass found a link.
+struct CcState {
+  unsigned long long list[2];
+  int largest;
+  int hooked;
+};
 
-template <int B>
-__global__ void k_cc_mngf_finish(GView v, int* __restrict__ mngf, Ctrl* __restrict__ ctrl,
-                                 const int* __restrict__ scratch) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (long long)v.nsplit * B) return;
-  const gbo_split sp = v.splits[gid / B];
-  const int r = (int)(gid % B);
-  int a = kINF;
-  for (int q = 0; q < sp.nslots; ++q) a = min(a, scratch[(size_t)(sp.slot0 + q) * B + r]);
-  const long long row = (long long)sp.row * B + r;
-  if (row < v.nrows && a < mngf[row]) mngf[row] = a;
-}
-
-__global__ void k_cc_hook(int* __restrict__ f, const int* __restrict__ mngf, int n, Ctrl* ctrl) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < n;
-       u += (long long)gridDim.x * blockDim.x) {
-    const int m = mngf[u];
-    const int fu = f[u];
-    if (m < fu) atomicMin(f + fu, m);  // stochastic hooking f[f[u]] <- mngf[u]
-  }
-}
-
-__global__ void k_cc_shortcut(int* __restrict__ f, const int* __restrict__ mngf,
-                              const int* __restrict__ gf, int n, Ctrl* ctrl) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < n;
-       u += (long long)gridDim.x * blockDim.x) {
-    const int m = min(mngf[u], gf[u]);  // aggressive hooking + shortcutting
-    if (m < f[u]) atomicMin(f + u, m);
-  }
-}
-
-__global__ void k_cc_grand(const int* __restrict__ f, int* __restrict__ gf, int n, Ctrl* ctrl) {
-  if (((volatile Ctrl*)ctrl)->done) return;
-  unsigned long long changed = 0;
-  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < n;
-       u += (long long)gridDim.x * blockDim.x) {
-    const int g2 = f[f[u]];
-    if (g2 != gf[u]) {
-      gf[u] = g2;
-      ++changed;
-    }
-  }
-  block_add_u64(changed, &ctrl->count);
-  close_iteration(ctrl, [](volatile Ctrl* c, int it) {
-    return c->count == 0ull || it >= c->max_iter;
-  });
-}
-
-__global__ void k_cc_init(int* f, int* gf, int* mngf, int n, Ctrl* ctrl, int max_iter) {
+// Every vertex under its first neighbour where that is lower (a forest: links
+// go down), so the first edge costs no atomic.
+__global__ void k_cc_init(GatherList gl, int* __restrict__ comp, CcState* __restrict__ st) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long k = i; k < n; k += stride) {
-    f[k] = (int)k;
-    gf[k] = (int)k;
-    mngf[k] = (int)k;
-  }
   if (i == 0) {
-    ctrl->iter = 0;
-    ctrl->done = 0;
-    ctrl->ticket = 0;
-    ctrl->max_iter = max_iter;
-    ctrl->count = 0;
-    ctrl->err = 0;
-    ctrl->last_err = 0;
-    ctrl->bar_err = 0u;
+    st->list[0] = st->list[1] = 0ull;
+    st->hooked = 0;
   }
+  for (long long v = i; v < gl.nrows; v += (long long)gridDim.x * blockDim.x) {
+    const long long b = gl.ptr[v], e = gl.ptr[v + 1];
+    comp[v] = e > b ? min((int)v, gl.col[b]) : (int)v;
+  }
+}
+
+// An edge between flattened trees: the higher root goes under the lower one.
+// Edges that meet at one root keep the lowest link only -- there is no retry to
+// contend for, and a link lost here is found again by a later pass.
+__device__ __forceinline__ bool cc_hook(int* comp, int u, int v) {
+  const int x = __ldca(comp + u), y = __ldca(comp + v);
+  const int hi = max(x, y), lo = min(x, y);
+  if (hi != lo && __ldca(comp + hi) > lo) atomicMin(comp + hi, lo);
+  return hi != lo;
+}
+
+// One more edge per vertex: neighbour `pick` of its list, from the end when
+// negative.
+__global__ void k_cc_hook(GatherList gl, int* comp, int pick) {
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < gl.nrows;
+       v += (long long)gridDim.x * blockDim.x) {
+    const long long b = gl.ptr[v], e = gl.ptr[v + 1];
+    const long long q = pick < 0 ? e + pick : b + pick;
+    if (q > b && q < e) cc_hook(comp, (int)v, gl.col[q]);
+  }
+}
+
+// Every vertex directly under its root (roots do not move meanwhile): each
+// thread doubles its own vertex's pointer, reading from L2 what the others
+// have doubled so far, so a path of d vertices takes about log d turns (read
+// through L1 it is walked: a mesh's paths of 1,000 took 392 us, now 34).
+__global__ void k_cc_compress(int* comp, int n, const CcState* __restrict__ if_hooked) {
+  if (if_hooked && !if_hooked->hooked) return;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    int p = __ldca(comp + v);
+    if (__ldca(comp + p) == p) continue;  // under a root already: popular roots stay in L1
+    for (int g = __ldcg(comp + p); g != p; g = __ldcg(comp + p)) {
+      __stcg(comp + v, g);
+      p = g;
+    }
+  }
+}
+
+// The labels: every vertex's root, each vertex written by its own thread only.
+__global__ void k_cc_labels(int* comp, int n, const CcState* __restrict__ st) {
+  if (!st->hooked) return;  // the trees are flat
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    int r = __ldca(comp + v);
+    for (int p = __ldca(comp + r); p != r; p = __ldca(comp + r)) r = p;
+    comp[v] = r;
+  }
+}
+
+// The most frequent label among the ends of kCcSamples set bits (a wrong guess
+// costs time only).
+__global__ void __launch_bounds__(kCcSamples) k_cc_sample(GatherList gl, const int* __restrict__ comp,
+                                                          CcState* __restrict__ st) {
+  __shared__ int lab[kCcSamples];
+  __shared__ unsigned best;
+  const int t = (int)threadIdx.x;
+  const unsigned h = ((unsigned)t + 1u) * 2654435761u;
+  const int mine = gl.nnz > 0 ? comp[gl.col[(long long)(((unsigned long long)h * (unsigned long long)gl.nnz) >> 32)]] : -1;
+  lab[t] = mine;
+  if (t == 0) best = 0u;
+  __syncthreads();
+  unsigned c = 0;
+#pragma unroll 16
+  for (int q = 0; q < kCcSamples; ++q) c += lab[q] == mine;
+  if (mine >= 0) atomicMax(&best, (c << 16) | (unsigned)t);  // count, then any of its holders
+  __syncthreads();
+  if (t == 0) st->largest = best ? lab[best & 0xffffu] : -1;
+}
+
+// Vertices outside the sampled component: all their edges.  Short rows a lane
+// each, others by the warp, rows past kCcChunk listed for k_cc_long.  The
+// first pass (LINK = false) hooks without retries; where it meets no edge
+// between two trees, the labels are final and the kernels behind it return
+// at once.  Else the second one (after a compress) links every edge for good.
+template <bool LINK>
+__device__ __forceinline__ bool cc_edge(int* comp, int u, int v) {
+  if (!LINK) return cc_hook(comp, u, v);
+  cc_link(comp, u, v);
+  return false;
+}
+
+template <bool LINK>
+__global__ void __launch_bounds__(kTPB) k_cc_rest(GatherList gl, int* comp, CcState* st, long long* list) {
+  if (LINK && !st->hooked) return;
+  const unsigned lane = threadIdx.x & 31;
+  // the second pass after the compress: the sampled component's label now
+  const int sampled = st->largest;
+  const int largest = LINK && sampled >= 0 ? comp[sampled] : sampled;
+  const long long nwarps = warps_total();
+  bool found = false;
+  for (long long base = warp_global() * 32; base < gl.nrows; base += nwarps * 32) {
+    const long long v = base + lane;
+    long long b = 0, e = 0;
+    if (v < gl.nrows && comp[v] != largest) {
+      b = gl.ptr[v];
+      e = gl.ptr[v + 1];
+    }
+    if (e - b > kCcChunk) {
+      const unsigned long long chunks = (unsigned long long)((e - b + kCcChunk - 1) / kCcChunk);
+      const unsigned long long old = atomicAdd(&st->list[LINK], (1ull << kListShift) | chunks);
+      const long long q = (long long)(old >> kListShift);
+      list[2 * q] = (long long)(old & kListMask);
+      list[2 * q + 1] = v;
+      e = b;
+    }
+    if (e - b <= kCcShort)
+      for (long long q = b; q < e; ++q) found |= cc_edge<LINK>(comp, (int)v, gl.col[q]);
+    for (unsigned m = __ballot_sync(0xffffffffu, e - b > kCcShort); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const long long rb = __shfl_sync(0xffffffffu, b, l), re = __shfl_sync(0xffffffffu, e, l);
+      for (long long q = rb + lane; q < re; q += 32) found |= cc_edge<LINK>(comp, (int)(base + l), gl.col[q]);
+    }
+  }
+  if (found) st->hooked = 1;
+}
+
+template <bool LINK>
+__global__ void __launch_bounds__(kTPB) k_cc_long(GatherList gl, int* comp, CcState* st,
+                                                  const long long* __restrict__ list) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned long long acc = st->list[LINK];
+  const long long nl = (long long)(acc >> kListShift), total = (long long)(acc & kListMask);
+  bool found = false;
+  for (long long q = warp_global(); q < total; q += warps_total()) {
+    long long lo = 0, hi = nl - 1;  // the row of chunk q
+    while (lo < hi) {
+      const long long mid = (lo + hi + 1) >> 1;
+      if (list[2 * mid] <= q) lo = mid;
+      else hi = mid - 1;
+    }
+    const long long v = list[2 * lo + 1];
+    const long long b = gl.ptr[v] + (q - list[2 * lo]) * kCcChunk, e = min(b + kCcChunk, gl.ptr[v + 1]);
+    for (long long p = b + lane; p < e; p += 32) found |= cc_edge<LINK>(comp, (int)v, gl.col[p]);
+  }
+  if (found) st->hooked = 1;
 }
 
 // ================================================================ host
@@ -2026,48 +2071,50 @@ int ppr_backward_impl(gbo_graph* g, const float* d_w, float alpha, float tol, in
   return GBO_OK;
 }
 
-template <int B>
 int cc_impl(gbo_graph* g, int32_t* d_label, int* h_iters, cudaStream_t s) {
   AlgoState* a = nullptr;
   GBO_TRY(get_state(g, &a));
-  GBO_TRY(ensure_vec_i32(g, &a->f));
-  GBO_TRY(ensure_vec_i32(g, &a->gf));
-  GBO_TRY(ensure_vec_i32(g, &a->mngf));
-  GView v = view_of(g);
-  int *f = a->f, *gf = a->gf, *mngf = a->mngf;
-  Ctrl* ctrl = a->ctrl;
-  int* scratch = (int*)a->scratch;
+  GBO_TRY(build_gather(g, s));
+  const GatherList gl = gather_of(g);
   const int n = g->nrows;
-  // 32x32 ROW graphs take the neighbours' minimum over their row-word slices
-  if (B == 32 && g->layout == GBO_LAYOUT_ROW) GBO_TRY(build_rws(g, s));
-  const bool rws = B == 32 && g->layout == GBO_LAYOUT_ROW && g->rws_head != nullptr;
-  if (rws) v = view_of(g);
-  const unsigned gi = rws ? grid_persistent(k_cc_mngf_rws, g->nbr) : grid_items_persistent(k_cc_mngf<B>, g->nitems, B);
-  const unsigned gc = rws && g->rws_nchunk > 0 ? grid_persistent(k_cc_mngf_chunks, g->rws_nchunk) : 0u;
-  const unsigned gs = blocks_for((long long)g->nsplit * B, kTPB);
-  const unsigned gv = grid_vertex(n);
-  GBO_TRY(get_exec(a, A_CC, nullptr, [&](cudaStream_t cs, int k, int* nl) -> int {
-    if (rws) {
-      if (g->nitems > 0) k_cc_mngf_rws<<<gi, kTPB, 0, cs>>>(v, gf, mngf, ctrl);
-      if (gc > 0) k_cc_mngf_chunks<<<gc, kTPB, 0, cs>>>(v, gf, mngf, ctrl);
-      *nl += (g->nitems > 0) + (gc > 0) + 3;
-    } else {
-      if (g->nitems > 0) k_cc_mngf<B><<<gi, kTPB, 0, cs>>>(v, gf, mngf, ctrl, scratch);
-      *nl += (g->nitems > 0) + (g->nsplit > 0) + 3;
-      if (g->nsplit > 0) k_cc_mngf_finish<B><<<gs, kTPB, 0, cs>>>(v, mngf, ctrl, scratch);
+  if (!a->cc) {  // the state, then room for every row that can be long
+    const size_t nb = sizeof(CcState) + sizeof(long long) * 2 * (size_t)(gl.nnz / kCcChunk + 1);
+    GBO_CUDA_TRY(cudaMalloc(&a->cc, nb));
+    g->device_bytes += (long long)nb;
+  }
+  auto* st = static_cast<CcState*>(a->cc);
+  auto* list = reinterpret_cast<long long*>(st + 1);
+  a->step_ms.clear();
+  a->stats_pending = false;
+  a->coop_run = false;
+  a->replays = 0;
+  a->launches = 0;
+  a->h_ctrl->iter = 0;
+  if (n > 0) {
+    const unsigned gv = grid_vertex(n);
+    const bool longs = gl.nnz > kCcChunk;
+    const unsigned gc = longs ? grid_persistent(k_cc_long<true>, gl.nnz / kCcChunk + 1) : 0u;
+    k_cc_init<<<gv, kTPB, 0, s>>>(gl, d_label, st);
+    for (const int pick : {-1, 1}) {
+      k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr);
+      k_cc_hook<<<gv, kTPB, 0, s>>>(gl, d_label, pick);
     }
-    k_cc_hook<<<gv, kTPB, 0, cs>>>(f, mngf, n, ctrl);
-    k_cc_shortcut<<<gv, kTPB, 0, cs>>>(f, mngf, gf, n, ctrl);
-    k_cc_grand<<<gv, kTPB, 0, cs>>>(f, gf, n, ctrl);
+    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr);
+    k_cc_sample<<<1, kCcSamples, 0, s>>>(gl, d_label, st);
+    k_cc_rest<false><<<gv, kTPB, 0, s>>>(gl, d_label, st, list);
+    if (longs) k_cc_long<false><<<gc, kTPB, 0, s>>>(gl, d_label, st, list);
+    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, st);
+    k_cc_rest<true><<<gv, kTPB, 0, s>>>(gl, d_label, st, list);
+    if (longs) k_cc_long<true><<<gc, kTPB, 0, s>>>(gl, d_label, st, list);
+    k_cc_labels<<<gv, kTPB, 0, s>>>(d_label, n, st);
     GBO_CUDA_TRY(cudaGetLastError());
-    return GBO_OK;
-  }));
-  const int max_iter = n + 2;
-  k_cc_init<<<gv, kTPB, 0, s>>>(f, gf, mngf, n, ctrl, max_iter);
-  GBO_CUDA_TRY(cudaGetLastError());
-  GBO_TRY(run_until_done(a, A_CC, s, max_iter, h_iters));
-  if (n > 0)
-    GBO_CUDA_TRY(cudaMemcpyAsync(d_label, f, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s));
+    a->launches = 11 + (longs ? 2 : 0);
+    a->h_ctrl->iter = 2;  // the sampled edges, the rest
+  }
+  if (h_iters) {
+    GBO_CUDA_TRY(cudaStreamSynchronize(s));
+    *h_iters = a->h_ctrl->iter;
+  }
   return GBO_OK;
 }
 
@@ -2199,9 +2246,7 @@ void free_algo_state(gbo_graph* g) {
   cudaFree(a->dist);
   cudaFree(a->pr);
   cudaFree(a->prs);
-  cudaFree(a->f);
-  cudaFree(a->gf);
-  cudaFree(a->mngf);
+  cudaFree(a->cc);
   cudaFree(a->acc64);
   cudaFree(a->pr_part);
   cudaFree(a->push_list);
@@ -2270,7 +2315,7 @@ extern "C" int gbo_cc(const gbo_graph* gc, int32_t* d_label, int* h_iters, gbo_s
   gbo_graph* g = const_cast<gbo_graph*>(gc);
   if (!d_label && g->nrows > 0) return fail(GBO_ERR_INVALID, "label is NULL");
   int st = GBO_OK;
-  ALGO_DISPATCH_B(g->b, st = cc_impl<B>(g, d_label, h_iters, as_stream(stream)));
+  st = cc_impl(g, d_label, h_iters, as_stream(stream));
   return st;
 }
 
