@@ -126,6 +126,54 @@ __global__ void k_list_parts(const long long* __restrict__ ptr, int nrows, int n
   part[i] = GatherPart{(int)a0, (int)(a1 - a0), a0 < nrows && ptr[a0] < i * kPartItems - a0 ? 1 : 0, 0};
 }
 
+// Long rows: 1 and the number of chunks where a row is one, else 0.
+__global__ void k_long_flags(const int* __restrict__ len, int nrows, int* __restrict__ flag, int* __restrict__ chunks) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nrows) return;
+  const bool l = len[i] > kLongRow;
+  flag[i] = l;
+  chunks[i] = l ? (len[i] + kLongChunk - 1) / kLongChunk : 0;
+}
+
+__global__ void k_long_fill(const int* __restrict__ len, int nrows, const int* __restrict__ at,
+                            const int* __restrict__ chunk_at, int* __restrict__ row, int* __restrict__ chunk0) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nrows) return;
+  if (len[i] > kLongRow) {
+    row[at[i]] = (int)i;
+    chunk0[at[i]] = chunk_at[i];
+  }
+  if (i == 0) chunk0[at[nrows]] = chunk_at[nrows];
+}
+
+int build_long(gbo_graph* g, const int* len, cudaStream_t s) {
+  const size_t n = (size_t)g->nrows;
+  int* tmp = nullptr;  // {flags, chunks, their prefix sums}
+  GBO_CUDA_TRY(pool_malloc_async(&tmp, sizeof(int) * (4 * n + 2) + sizeof(long long) * 3, s));
+  int *flag = tmp, *chunks = flag + n, *at = chunks + n, *chunk_at = at + n + 1;
+  auto* tot = reinterpret_cast<long long*>((reinterpret_cast<uintptr_t>(chunk_at + n + 1) + 7) & ~(uintptr_t)7);
+  const int st = [&]() -> int {
+    k_long_flags<<<blocks_for(g->nrows, 256), 256, 0, s>>>(len, g->nrows, flag, chunks);
+    GBO_TRY(exclusive_scan_i32(flag, at, g->nrows, tot, s));
+    GBO_TRY(exclusive_scan_i32(chunks, chunk_at, g->nrows, tot + 1, s));
+    long long h[2] = {0, 0};
+    const cudaError_t e = read_back(h, tot, sizeof(h), s);
+    if (e != cudaSuccess) return fail_cuda(e, "long rows");
+    if (h[1] > 2147483647ll) return fail(GBO_ERR_OVERFLOW, "row lists: too many entries");
+    GBO_CUDA_TRY(cudaMalloc(&g->gl_long_row, sizeof(int) * (size_t)(h[0] > 0 ? h[0] : 1)));
+    GBO_CUDA_TRY(cudaMalloc(&g->gl_long_chunk0, sizeof(int) * (size_t)(h[0] + 1)));
+    k_long_fill<<<blocks_for(g->nrows, 256), 256, 0, s>>>(len, g->nrows, at, chunk_at, g->gl_long_row,
+                                                          g->gl_long_chunk0);
+    GBO_CUDA_TRY(cudaGetLastError());
+    g->gl_nlong = (int)h[0];
+    g->gl_nlchunk = (int)h[1];
+    g->device_bytes += 4LL * (2 * h[0] + 1);
+    return GBO_OK;
+  }();
+  cudaFreeAsync(tmp, s);
+  return st;
+}
+
 template <int B>
 int build_impl(gbo_graph* g, int* cnt, int* len, int* first, long long* tot, cudaStream_t s) {
   const GView v = view_of(g);
@@ -148,6 +196,7 @@ int build_impl(gbo_graph* g, int* cnt, int* len, int* first, long long* tot, cud
   k_list_parts<<<blocks_for(parts, 256), 256, 0, s>>>(g->gl_ptr, v.nrows, (int)parts,
                                                       static_cast<GatherPart*>(g->gl_part));
   GBO_CUDA_TRY(cudaGetLastError());
+  GBO_TRY(build_long(g, len, s));
   g->gl_nparts = (int)parts;
   g->gl_nnz = nnz;
   g->device_bytes += 4LL * nnz + 8LL * (v.nrows + 1) + (long long)sizeof(GatherPart) * parts;
@@ -160,6 +209,12 @@ void free_gather(gbo_graph* g) {
   cudaFree(g->gl_ptr);
   cudaFree(g->gl_col);
   cudaFree(g->gl_part);
+  cudaFree(g->gl_long_row);
+  cudaFree(g->gl_long_chunk0);
+  g->gl_long_row = nullptr;
+  g->gl_long_chunk0 = nullptr;
+  g->gl_nlong = 0;
+  g->gl_nlchunk = 0;
   g->gl_ptr = nullptr;
   g->gl_col = nullptr;
   g->gl_part = nullptr;
@@ -209,6 +264,10 @@ GatherList gather_of(const gbo_graph* g) {
   gl.nnz = g->gl_nnz;
   gl.nrows = g->nrows;
   gl.nparts = g->gl_nparts;
+  gl.nlong = g->gl_nlong;
+  gl.nchunk = g->gl_nlchunk;
+  gl.long_row = g->gl_long_row;
+  gl.long_chunk0 = g->gl_long_chunk0;
   return gl;
 }
 

@@ -48,7 +48,28 @@ struct GatherList {
   long long nnz = 0;
   int nrows = 0;
   int nparts = 0;
+  // rows of more than kLongRow set bits, for kernels that give a row a warp:
+  // chunks of kLongChunk set bits, long row q's from chunk0[q] on
+  int nlong = 0;
+  int nchunk = 0;
+  const int* __restrict__ long_row = nullptr;
+  const int* __restrict__ long_chunk0 = nullptr;
 };
+
+constexpr int kLongRow = 256;
+constexpr int kLongChunk = 256;
+
+// Index among the long rows of the last one whose key (its row, or its first
+// chunk) is at most x.
+__device__ __forceinline__ int long_index(const int* __restrict__ key, int n, int x) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (key[mid] <= x) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
 
 // Build g's row lists if needed (synchronises `s` when it does).
 int build_gather(gbo_graph* g, cudaStream_t s);

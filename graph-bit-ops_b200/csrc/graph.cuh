@@ -62,6 +62,10 @@ struct gbo_graph {
   void* gl_part = nullptr;      // gl_nparts parts (GatherPart)
   long long gl_nnz = 0;
   int gl_nparts = -1;           // -1: not built
+  int gl_nlong = 0;             // rows of more than kLongRow set bits,
+  int gl_nlchunk = 0;           // their chunks (at most kLongChunk set bits each)
+  int* gl_long_row = nullptr;   // gl_nlong rows, ascending
+  int* gl_long_chunk0 = nullptr;  // gl_nlong + 1: each one's first chunk
   int last_run_ms = 0;     // 1: the last traversal was a multi-source BFS
   bool tc_mma = false;     // GBO_FLAG_TC_MMA: dense 32x32 mask tiles on the 1-bit MMA
   bool owns_outdeg = true;

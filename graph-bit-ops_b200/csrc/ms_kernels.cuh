@@ -16,6 +16,7 @@
 // visited rows, levels and both bit vectors.
 #pragma once
 
+#include "gather.cuh"
 #include "scan.cuh"
 
 namespace gbo {
@@ -65,6 +66,9 @@ struct Args {
   // rows (rws_nlong x KW words, zero between levels; k_long_chunks ORs into
   // them, k_step_rws reads them, a memset after the step clears them)
   uint32_t* long_acc = nullptr;
+  // wide frontier rows (k > 64): the row lists; long_acc then holds nlong x KW
+  // words (k_wide_long, k_step_wide)
+  GatherList gl;
 };
 
 // Address of the level of (vertex i, source s) in either layout.
@@ -570,6 +574,230 @@ __global__ void __launch_bounds__(kTPB, 6) k_step_rws(Args a) {
   }
 }
 
+// Pull step for wide frontier rows (KW = 4 to 32 words, k > 64) over the row
+// lists: a block per block row, its warps over the rows.  At KW = 32 a warp
+// takes a row: it reads 32 of its columns at once, keeps those whose vertex is
+// in the frontier in a small list and ORs their frontier rows, one 128-byte
+// load of the whole warp each.  Narrower rows go to groups of KW lanes (8 at
+// KW = 4), so that the instructions of a row are shared by two to four.  A
+// row leaves once every active source has reached it.  Rows past kLongRow come
+// from k_wide_long, a warp per chunk.
+//
+// Bound by the frontier rows' bytes from L2 at KW = 32, by instructions at 4.
+// k = 1,000 on R-MAT 17 (3.6 M set bits): 1.26 and 1.41 ms for the two dense
+// levels when the (row, vertex) pairs of the tiles' words were listed and
+// OR-ed with shared-memory atomics, MEASURE now.
+constexpr int kWideList = 64;
+
+template <int KW>
+__device__ __forceinline__ uint32_t or_slots(uint32_t v) {
+#pragma unroll
+  for (int o = KW; o < 32; o <<= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// This lane's column among [b, e) and whether its vertex is in the frontier.
+__device__ __forceinline__ int wide_column(const int* __restrict__ col, long long b, long long e, unsigned lane) {
+  return b + lane < e ? col[b + lane] : -1;
+}
+__device__ __forceinline__ bool wide_in_front(const uint32_t* __restrict__ fb, int c) {
+  return c >= 0 && ((fb[c >> 5] >> (31 - (c & 31))) & 1u);
+}
+
+// OR of the frontier rows of columns [b, e), word lane % KW in every lane;
+// stops early once `have` and it cover `need` in every word.
+template <int KW>
+__device__ __forceinline__ uint32_t wide_gather(const uint32_t* __restrict__ F, const uint32_t* __restrict__ fb,
+                                                const int* __restrict__ col, long long b, long long e,
+                                                int* __restrict__ list, unsigned lane, uint32_t have, uint32_t need) {
+  constexpr int S = 32 / KW;
+  constexpr int U = KW >= 8 ? 8 : 32 / S;  // loads in flight per lane
+  const int w = (int)lane % KW, s = (int)lane / KW;
+  uint32_t acc = 0u;
+  int n = 0;  // queued columns (warp-uniform)
+  int c = wide_column(col, b, e, lane);
+  for (long long p = b; p < e; p += 32) {
+    const int cn = wide_column(col, p + 32, e, lane);
+    const bool f = wide_in_front(fb, c);
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    if (f) list[n + __popc(m & ((1u << lane) - 1u))] = c;
+    n += __popc(m);
+    c = cn;
+    if (n < 32 && p + 32 < e) continue;
+    __syncwarp();
+    for (int t = 0; t < n; t += S * U) {
+      uint32_t x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int q = t + u * S + s;
+        x[u] = q < n ? __ldg(F + (size_t)list[q] * KW + w) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc |= x[u];
+    }
+    n = 0;
+    acc = or_slots<KW>(acc);
+    if (__all_sync(0xffffffffu, ((have | acc) & need) == need)) break;
+    __syncwarp();
+  }
+  return acc;
+}
+
+// Long rows: a warp per chunk, its OR added to the row's long_acc words; a row
+// that its earlier chunks have covered is left.
+template <int KW>
+__global__ void __launch_bounds__(kTPB) k_wide_long(Args a) {
+  __shared__ int list_sh[kWarps][kWideList];
+  volatile int* c = a.ctl;
+  if (c[1]) return;
+  if (a.dir && (c[7] || c[6] == 1)) return;
+  const int lvl = c[0];
+  const uint32_t* __restrict__ F = a.F + (size_t)(lvl & 1) * a.fstride;
+  const uint32_t* __restrict__ fb = a.fbits + (size_t)(lvl & 1) * (a.v.nbr + 1);
+  const unsigned lane = threadIdx.x & 31;
+  const int w = (int)lane % KW;
+  const uint32_t need = src_mask(w, a.k) & (a.active ? a.active[w] : 0xffffffffu);
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < a.gl.nchunk; q += nwarps) {
+    const int l = long_index(a.gl.long_chunk0, a.gl.nlong, (int)q);
+    const int i = a.gl.long_row[l];
+    if ((a.vfull[i >> 5] >> (31 - (i & 31))) & 1u) continue;  // row finished
+    uint32_t* dst = a.long_acc + (size_t)l * KW + w;
+    const uint32_t have = a.V[(size_t)i * KW + w] | __ldcg(dst);
+    if (__all_sync(0xffffffffu, (have & need) == need)) continue;
+    const long long b = a.gl.ptr[i] + (q - a.gl.long_chunk0[l]) * kLongChunk;
+    const long long e = min(b + kLongChunk, a.gl.ptr[i + 1]);
+    const uint32_t acc = wide_gather<KW>(F, fb, a.gl.col, b, e, list_sh[threadIdx.x >> 5], lane, have, need);
+    if ((int)lane < KW && (acc & ~have)) atomicOr(dst, acc);
+    __syncwarp();
+  }
+}
+
+// Warps of a block: few where a row needs few, so that a late level -- most
+// block rows with a row or two still open -- keeps more block rows in flight.
+template <int KW>
+__host__ __device__ constexpr int wide_warps() {
+  return KW <= 8 ? 2 : KW == 16 ? 4 : 8;
+}
+
+template <int KW>
+__global__ void __launch_bounds__(wide_warps<KW>() * 32) k_step_wide(Args a) {
+  constexpr int kW = wide_warps<KW>();
+  __shared__ int list_sh[KW == 32 ? kW : 1][kWideList];
+  __shared__ int rows_sh[32];  // the open rows
+  __shared__ uint32_t any_sh[KW];
+  __shared__ uint32_t fword_sh, vword_sh;
+  __shared__ unsigned cnt_sh;
+  volatile int* c = a.ctl;
+  if (c[1]) return;
+  if (a.dir && (c[7] || c[6] == 1)) return;  // this slot's level ran as a push
+  const int lvl = c[0];
+  const int nbr = a.v.nbr, R = (int)blockIdx.x;
+  const uint32_t vrow = a.vfull[R];
+  uint32_t* fn = a.fbits + (size_t)((lvl + 1) & 1) * (nbr + 1) + R;
+  if (vrow == 0xffffffffu) {
+    if (threadIdx.x == 0) *fn = 0u;
+    return;
+  }
+  const uint32_t* __restrict__ F = a.F + (size_t)(lvl & 1) * a.fstride;
+  const uint32_t* __restrict__ fb = a.fbits + (size_t)(lvl & 1) * (nbr + 1);
+  uint32_t* Fn = a.F + (size_t)((lvl + 1) & 1) * a.fstride;
+  const unsigned lane = threadIdx.x & 31;
+  constexpr int G = KW < 8 ? 8 : KW, S = G / KW;  // lanes of a row, slots
+  const uint32_t openm = ~vrow;                   // bit 31 - r: row r (padding rows are marked finished)
+  const int nopen = __popc(openm);
+  const int wib = (int)(threadIdx.x >> 5);
+  const int grp = (int)lane / G, w = (int)lane % KW, slot = (int)lane % G / KW;
+  if (threadIdx.x < KW) any_sh[threadIdx.x] = 0u;
+  if (threadIdx.x < 32 && ((openm >> (31 - threadIdx.x)) & 1u))
+    rows_sh[__popc(openm & ~(0xffffffffu >> threadIdx.x))] = (int)threadIdx.x;
+  if (threadIdx.x == 0) {
+    fword_sh = 0u;
+    vword_sh = vrow;
+    cnt_sh = 0u;
+  }
+  __syncthreads();
+  const uint32_t mask = src_mask(w, a.k), need = mask & (a.active ? a.active[w] : 0xffffffffu);
+  unsigned cnt = 0;
+  uint32_t anyw = 0u;
+  constexpr unsigned kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+#pragma unroll 1
+  for (int q0 = wib * (32 / G); q0 < nopen; q0 += kW * (32 / G)) {
+    const bool open = q0 + grp < nopen;
+    const int r = open ? rows_sh[q0 + grp] : 0;
+    const int i = R * 32 + r;
+    const size_t o = (size_t)i * KW + w;
+    uint32_t have = 0u, acc = 0u;
+    long long b = 0, e = 0;
+    if (open) {
+      have = a.V[o];
+      b = a.gl.ptr[i];
+      e = a.gl.ptr[i + 1];
+    }
+    const bool lng = e - b > kLongRow;
+    if (lng) acc = a.long_acc[(size_t)long_index(a.gl.long_row, a.gl.nlong, i) * KW + w];
+    if constexpr (KW == 32) {
+      if (!lng) acc = wide_gather<KW>(F, fb, a.gl.col, b, e, list_sh[wib], lane, have, need);
+    } else {
+      bool go = e > b && !lng;
+      int c = go ? wide_column(a.gl.col, b, e, lane % G) : -1;
+      for (long long p = b; __any_sync(0xffffffffu, go); p += G) {
+        const int cc = go && wide_in_front(fb, c) ? c : -1;
+        c = go ? wide_column(a.gl.col, p + G, e, lane % G) : -1;
+#pragma unroll
+        for (int t0 = 0; t0 < KW; t0 += KW < 8 ? KW : 8) {
+          constexpr int U = KW < 8 ? KW : 8;
+          uint32_t x[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int q = __shfl_sync(0xffffffffu, cc, grp * G + (t0 + u) * S + slot);
+            x[u] = q >= 0 ? __ldg(F + (size_t)q * KW + w) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) acc |= x[u];
+        }
+#pragma unroll
+        for (int o = KW; o < G; o <<= 1) acc |= __shfl_xor_sync(0xffffffffu, acc, o);
+        const unsigned cov = __ballot_sync(0xffffffffu, ((have | acc) & need) == need) >> (grp * G);
+        go = go && p + G < e && (cov & kGroup) != kGroup;
+      }
+    }
+    const uint32_t nw = open ? acc & ~have & mask : 0u, vn = have | nw;
+    const unsigned news = __ballot_sync(0xffffffffu, nw != 0u && slot == 0);
+    const bool any = ((news >> (grp * G)) & kGroup) != 0u;
+    const unsigned cov = __ballot_sync(0xffffffffu, (vn & need) == need) >> (grp * G);
+    if (any && slot == 0) {
+      Fn[o] = nw;  // only rows marked in fbits are ever read
+      a.V[o] = vn;
+      cnt += __popc(nw);
+      anyw |= nw;
+    }
+    // levels of the new pairs: a word's sources by consecutive lanes
+    for (unsigned m = news; m; m &= m - 1) {
+      const int t = __ffs(m) - 1;
+      const int it = R * 32 + rows_sh[q0 + t / G];
+      if ((__shfl_sync(0xffffffffu, nw, t) >> lane) & 1u) a.levels[level_index(a, it, t % KW * 32 + (int)lane)] = lvl + 1;
+    }
+    if ((int)lane % G == 0 && any) atomicOr(&fword_sh, 1u << (31 - r));
+    if ((int)lane % G == 0 && open && (cov & kGroup) == kGroup) atomicOr(&vword_sh, 1u << (31 - r));
+    __syncwarp();
+  }
+  if (anyw) atomicOr(any_sh + w, anyw);
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0 && cnt) atomicAdd(&cnt_sh, cnt);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *fn = fword_sh;
+    a.vfull[R] = vword_sh;
+    if (cnt_sh) atomicAdd(reinterpret_cast<unsigned long long*>(a.ctl + 4), (unsigned long long)cnt_sh);
+  }
+  if (a.slot_any && threadIdx.x < KW && any_sh[threadIdx.x]) {
+    // most columns are marked early in a level, so few atomics reach one address
+    const uint32_t cur = __ldcg(a.slot_any + threadIdx.x);
+    if (any_sh[threadIdx.x] & ~cur) atomicOr(a.slot_any + threadIdx.x, any_sh[threadIdx.x]);
+  }
+}
+
 // Block count of a level and its close: the last block to arrive (arrival
 // ticket in ctl[2], no waiting) advances the level, stops at a zero count or
 // the iteration cap and, with dir, picks the next level's mode; `pushed`
@@ -591,6 +819,11 @@ __device__ __forceinline__ void close_level(const Args& a, unsigned long long cn
     last = atomicAdd(reinterpret_cast<unsigned*>(a.ctl + 2), 1u) == gridDim.x - 1;
   }
   __syncthreads();
+  if (last && a.retire && a.active && a.slot_any && threadIdx.x < (unsigned)((a.k + 31) / 32)) {
+    __threadfence();
+    a.active[threadIdx.x] &= __ldcg(a.slot_any + threadIdx.x);  // a thread per word (16 us by one thread at 32 words)
+    a.slot_any[threadIdx.x] = 0u;
+  }
   if (last && threadIdx.x == 0) {
     __threadfence();
     volatile unsigned long long* vc = count;
@@ -605,13 +838,6 @@ __device__ __forceinline__ void close_level(const Args& a, unsigned long long cn
     *vc = 0ull;
     a.ctl[2] = 0;
     if (stop) c[1] = 1;
-    if (a.retire && a.active && a.slot_any) {
-      volatile uint32_t* any = a.slot_any;
-      for (int w = 0; w < (a.k + 31) / 32; ++w) {
-        a.active[w] &= any[w];
-        any[w] = 0u;
-      }
-    }
     __threadfence();
   }
 }

@@ -8,6 +8,7 @@
 // Multi-seed BFS (gbo_bfs_multi) reuses the single-frontier BFS loop of
 // algo.cu with several level-0 vertices; on a block-diagonal union of graphs
 // with one seed per graph it is every graph's own BFS in one traversal.
+#include <algorithm>
 #include <vector>
 
 #include "ms_kernels.cuh"
@@ -29,7 +30,8 @@ struct MsState {
   uint32_t* split_acc = nullptr;
   int* slot_split = nullptr;
   uint32_t* push_acc = nullptr;  // nbr * 32 * kw (push levels; k <= 64 on symmetric graphs)
-  uint32_t* long_acc = nullptr;  // rws_nlong * 2 (slice steps, k <= 64)
+  uint32_t* long_acc = nullptr;  // long rows' gathered frontier rows: rws_nlong * 2 (slice
+  size_t long_words = 0;         // steps, k <= 64) or gl_nlong * kw (row lists, wider)
   uint32_t* active = nullptr;    // 32 words: source columns still traversing
   uint32_t* slot_any = nullptr;  // 32 words: columns with a new vertex in the level
   int* srcs = nullptr;
@@ -85,6 +87,7 @@ ms::Args make_args(gbo_graph* g, MsState& m, int32_t* d_levels, int k, int level
   a.dir = a.push_thr > 0 ? 1 : 0;
   a.push_acc = m.push_acc;
   a.long_acc = m.long_acc;
+  if (m.kw > 2) a.gl = gather_of(g);
   return a;
 }
 
@@ -92,12 +95,12 @@ template <int KW>
 int ms_capture(gbo_graph* g, MsState& m, int32_t* d_levels, int k, int level_group) {
   const ms::Args a = make_args(g, m, d_levels, k, level_group);
   // k <= 64 on a graph with row-word slices: the pull step walks rows
-  // (k_step_rws, whole block rows: no split partials for the finish kernel);
-  // wider frontier rows go through the tiles (k_step), which measured 2x
-  // faster than walking the slices at k = 256 and 1024 on R-MAT 21
+  // (k_step_rws); wider frontier rows walk the row lists (k_step_wide).  Both
+  // take whole block rows: no split partials for the finish kernel
   const bool rws = KW <= 2 && g->rws_head != nullptr;
+  const bool wide = KW > 2;
   ms::Args af = a;
-  if (rws) af.v.nsplit = 0;
+  if (rws || wide) af.v.nsplit = 0;
   const unsigned gi = rws ? blocks_for_warps(g->nbr > 0 ? g->nbr : 1, ms::kWarps)
                           : blocks_for_warps(g->nitems, ms::kWarps);
   const unsigned gs = blocks_for_warps(af.v.nsplit > 0 ? af.v.nsplit : 1, ms::kWarps);
@@ -130,7 +133,12 @@ int ms_capture(gbo_graph* g, MsState& m, int32_t* d_levels, int k, int level_gro
         if (rws && g->rws_nchunk > 0)
           cudaMemsetAsync(m.long_acc, 0, sizeof(uint32_t) * (size_t)g->rws_nlong * KW, m.cap);
       } else {
-        ms::k_step<KW><<<gi, ms::kTPB, 0, m.cap>>>(a);
+        if (g->gl_nlchunk > 0)
+          ms::k_wide_long<KW><<<std::min(blocks_for_warps(g->gl_nlchunk, ms::kWarps), (unsigned)num_sms() * 8u),
+                                ms::kTPB, 0, m.cap>>>(a);
+        ms::k_step_wide<KW><<<(unsigned)g->nbr, ms::wide_warps<KW>() * 32, 0, m.cap>>>(a);
+        if (g->gl_nlchunk > 0)
+          cudaMemsetAsync(m.long_acc, 0, sizeof(uint32_t) * (size_t)g->gl_nlong * KW, m.cap);
       }
     }
     if (a.dir) ms::k_finish<KW><<<gs, ms::kTPB, 0, m.cap>>>(af);
@@ -174,11 +182,7 @@ int msbfs_impl(gbo_graph* g, MsState& m, const int* h_srcs, int k, int32_t* d_le
     GBO_CUDA_TRY(cudaMalloc(&m.active, sizeof(uint32_t) * 64));
     m.slot_any = m.active + 32;
   }
-  if (!m.long_acc && g->rws_head) {  // slice steps: frontier rows of up to 2 words
-    const size_t lw = (size_t)(g->rws_nlong > 0 ? g->rws_nlong : 1) * 2;
-    GBO_CUDA_TRY(cudaMalloc(&m.long_acc, sizeof(uint32_t) * lw));
-    GBO_CUDA_TRY(cudaMemsetAsync(m.long_acc, 0, sizeof(uint32_t) * lw, s));
-  }
+  if (kw > 2) GBO_TRY(build_gather(g, s));
   if (kw != m.kw) {  // state sized for exactly kw words per vertex
     if (m.exec) cudaGraphExecDestroy(m.exec);
     m.exec = nullptr;
@@ -198,6 +202,15 @@ int msbfs_impl(gbo_graph* g, MsState& m, const int* h_srcs, int k, int32_t* d_le
       GBO_CUDA_TRY(cudaMalloc(&m.push_acc, sizeof(uint32_t) * pw));
       GBO_CUDA_TRY(cudaMemsetAsync(m.push_acc, 0, sizeof(uint32_t) * pw, s));
     }
+    const size_t lw = kw > 2 ? (size_t)std::max(g->gl_nlong, 1) * kw : (size_t)std::max(g->rws_nlong, 1) * 2;
+    if (lw > m.long_words) {
+      cudaFree(m.long_acc);
+      m.long_acc = nullptr;
+      m.long_words = 0;
+      GBO_CUDA_TRY(cudaMalloc(&m.long_acc, sizeof(uint32_t) * lw));
+      m.long_words = lw;
+    }
+    GBO_CUDA_TRY(cudaMemsetAsync(m.long_acc, 0, sizeof(uint32_t) * lw, s));
     m.kw = kw;
   }
   if (k > m.ksrc) {

@@ -1179,7 +1179,10 @@ extern "C" int gbo_server_create(const gbo_graph* gc, int bfs_slots, int ppr_slo
         S->live = static_cast<const uint32_t*>(lv);
       }
       {  // rounds of up to 64 slots walk the row-word slices
-        const int st = build_rws(g, S->s[0]);
+        int st = build_rws(g, S->s[0]);
+        // batches of more than 64 queries walk the row lists: built here, not
+        // by the worker thread beside a client's own calls on the graph
+        if (st == GBO_OK && kw > 2) st = build_gather(g, S->s[0]);
         if (st != GBO_OK) throw st;
         const size_t lw = (size_t)(g->rws_nlong > 0 ? g->rws_nlong : 1) * (size_t)std::min(kw, 2);
         cu(cudaMalloc(&S->long_acc, sizeof(uint32_t) * lw), "long_acc");

@@ -629,7 +629,8 @@ GBO_API int gbo_gen_er_batch(int count, int nmin, int nmax, double avg_degree,
  *       (readers, generators, CSR utilities) fails: the call returns
  *       GBO_ERR_NOMEM and leaves its output untouched;
  *   GBO_INJECT_REPLAY_CAP  (n >= 1) the iteration loops (BFS, SSSP,
- *       PageRank, PPR) run at most 8 n iterations and return GBO_ERR_TIMEOUT when the device has not finished by then;
+ *       PageRank, PPR) run at most 8 n iterations and return
+ *       GBO_ERR_TIMEOUT when the device has not finished by then;
  *   GBO_INJECT_SERVER_HOLD (n = 1) server workers admit no new query:
  *       submissions stay pending (queries already in flight finish);
  *   GBO_INJECT_BARRIER_SKIP (n >= 1) the next cooperative BFS launch (one
