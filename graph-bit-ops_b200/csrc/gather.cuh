@@ -56,6 +56,7 @@ struct GatherList {
   const int* __restrict__ long_chunk0 = nullptr;
 };
 
+constexpr int kShortRow = 8;
 constexpr int kLongRow = 256;
 constexpr int kLongChunk = 256;
 
@@ -73,6 +74,16 @@ __device__ __forceinline__ int long_index(const int* __restrict__ key, int n, in
 
 // Build g's row lists if needed (synchronises `s` when it does).
 int build_gather(gbo_graph* g, cudaStream_t s);
+
+// The lists' memory: from the library's pool, which has it mapped already when
+// a program makes one graph after another (cudaMalloc took 0.1-0.4 ms an
+// array).  Freeing waits for the device, as cudaFree does for its own memory.
+template <typename T>
+int list_alloc(T** p, size_t count, cudaStream_t s) {
+  GBO_CUDA_TRY(pool_malloc_async(p, sizeof(T) * (count > 0 ? count : 1), s));
+  return GBO_OK;
+}
+void lists_idle(const void* list);  // before cudaFree of a list
 GatherList gather_of(const gbo_graph* g);
 
 // Shared memory of a warp's part: the rows' sums (8 bytes each), the gathered

@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "bmv.cuh"
+#include "gather.cuh"
 
 namespace gbo {
 
@@ -108,6 +109,11 @@ void destroy(gbo_graph* g) {
   if (g->owns_outdeg) cudaFree(g->outdeg);
   cudaFree(g->perm);
   cudaFree(g->tile_row);
+  lists_idle(g->tc_ptr);
+  cudaFree(g->tc_ptr);
+  cudaFree(g->tc_col);
+  cudaFree(g->tc_unit);
+  cudaFree(g->tc_unit0);
   cudaFree(g->rowmask);
   cudaFree(g->rowword);
   cudaFree(g->item_wbase);

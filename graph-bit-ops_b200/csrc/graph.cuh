@@ -4,6 +4,8 @@
 
 #include "common.cuh"
 
+#include <mutex>
+
 // One warp-group work item: tiles [t0, t1) of block row `row`.  A block row
 // with more tiles than the chunk size is split into several items; those
 // write partial results into scratch `slot` and a reduce kernel combines
@@ -62,6 +64,18 @@ struct gbo_graph {
   void* gl_part = nullptr;      // gl_nparts parts (GatherPart)
   long long gl_nnz = 0;
   int gl_nparts = -1;           // -1: not built
+  bool gl_lower = false;        // no column past its row
+  std::mutex build_mu;          // one build of the lists at a time
+  bool gl_diag = false;         // some column equal to its row
+  bool gl_short = false;        // no row of more than kShortRow set bits
+  // triangle counting on a lower triangle: vertices ranked by falling degree,
+  // every edge in the list of its end of higher rank, and the warp units of
+  // the longer lists
+  long long* tc_ptr = nullptr;  // nrows + 1
+  int* tc_col = nullptr;
+  int* tc_unit = nullptr;       // the row of every unit
+  int* tc_unit0 = nullptr;      // every row's first unit (nrows + 1)
+  int tc_nunits = -1;           // -1: not built
   int gl_nlong = 0;             // rows of more than kLongRow set bits,
   int gl_nlchunk = 0;           // their chunks (at most kLongChunk set bits each)
   int* gl_long_row = nullptr;   // gl_nlong rows, ascending

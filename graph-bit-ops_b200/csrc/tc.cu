@@ -1,19 +1,41 @@
-// Triangle counting by masked binary SpGEMM on B2SR tiles.
+// Triangle counting: sum over the entries (i, k) of a lower triangle L of
+// |L_i & L_k|, the masked binary product of bmm32_sparse_masked_v5
+// (bsrbmm/bsrbmm.cu:1214-1265), which reduces into an int32 (overflows past
+// 2^31 triangles, bsrbmm/tc.cu:861-863).  The count is uint64.
 //
-// Reference: bmm32_sparse_masked_v5 (bsrbmm/bsrbmm.cu:1214-1265) computes
-// sum over mask tiles (I,K) of L of sum_r sum_c M[r][c] * (L L^T)[I*b+r][K*b+c],
-// looking up B = L^T tiles (col layout) by binary search, and reduces into an
-// int32 (overflows past 2^31 triangles, bsrbmm/tc.cu:861-863).
+// Lower triangles (every entry at or below the diagonal) are counted over
+// lists of neighbours: tiles of power-law graphs hold one or two bits, so a
+// pair of tiles costs two 32-byte sectors and a search for a bit of product.
+// A simple graph's triangles do not depend on which end an edge belongs to, so
+// once per graph the vertices are ranked by falling degree and every edge goes
+// to its end of lower degree, as the other end's rank: a list is at most
+// sqrt(2 edges) long, and hubs' lists are short (R-MAT 17: 252 M list entries
+// to look at instead of 405 M by vertex number, the longest list 329 instead
+// of 5,255).  Per list, a warp per kUnit entries looks up the lists of these
+// entries among the list itself: ranks below kBits -- nearly all of a
+// power-law graph's -- in an exact bitmap in shared memory, the others behind
+// a filter.  Where every row is a few entries long (meshes) the rows are
+// counted as they are, a lane each.  Diagonal entries add, per the formula
+// above, a term per entry in their column and their row's length.
 //
-// Here the L^T operand is never built: the col-layout tile (J,K) of L^T has
-// the same words as the row-layout tile (K,J) of L, so the intersection of
-// block rows I and K of L (restricted to block columns <= K) gives every
-// contributing pair.  One warp per mask tile probes the shorter of the two
-// sorted column lists into the longer with binary searches (32 probes per
-// step), and for each hit computes
-//   sum_r sum_{c in M_r} popc(A_(I,J)[r] & A_(K,J)[c])
-// with the K-tile rows broadcast by warp shuffles.  The count is uint64.
-#include "bmv.cuh"
+// Bound by the latency of the lists' reads from L2 at 32 warps an SM: kSide
+// lists are read side by side (1 / 2 / 4 / 8 of them: 716 / 561 / 491 / 681 us
+// at R-MAT 17, ef 16, b = 32; a bitmap of 16,384 ranks: 523; a hash of 1,024
+// entries in place of both: 1,171).  Tiles / lists, us, with the lists built:
+// R-MAT 17 2,679 / 483, ef 24 shuffled b = 16 5,261 / 921, R-MAT 20
+// 75,430 / 7,763, uniform of 100,003 vertices and 24 per vertex b = 8
+// 622 / 103, mesh of 10^6 vertices 121 / 42.  A graph's first call, building
+// included: 3,100 / 1,170, -, 76,000 / 11,600, 1,040 / 400, 530 / 210.
+//
+// Building costs 180 us and more however small the graph; the tiles of
+// kListTiles are counted in about 100 (uniform of 10,000 vertices, 65,764
+// tiles: 90, with lists 42, the first call 240; R-MAT of 20,001, 122,369:
+// 347, 54, 410).  Fewer tiles, tensor-core counts and matrices with an entry
+// above the diagonal keep the tile kernels, as does a first call under stream
+// capture, where nothing can be read back, or without memory for the lists.
+#include <algorithm>
+
+#include "gather.cuh"
 
 namespace gbo {
 
@@ -28,6 +50,268 @@ __device__ __forceinline__ int lower_bound_dev(const int* __restrict__ a, int lo
     else hi = mid;
   }
   return lo;
+}
+
+constexpr long long kListTiles = 1 << 16;
+constexpr int kUnit = 64;       // entries of a list that one warp goes through
+constexpr int kBits = 32768;    // ranks in a warp's bitmap
+constexpr int kPiece = 256;     // entries of a list looked up among at a time
+constexpr int kFilterBits = 2048;
+constexpr int kSide = 4;        // looked-up lists read side by side
+constexpr int kTcWarps = 8;     // warps of a block (5.3 KB of shared memory each)
+
+struct Lists {
+  const long long* __restrict__ ptr;
+  const int* __restrict__ col;
+  int n;
+};
+
+__global__ void k_count_cols(const int* __restrict__ col, long long nnz, int* __restrict__ deg) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (long long)gridDim.x * blockDim.x)
+    atomicAdd(deg + col[i], 1);
+}
+
+// Ranks by falling degree (row length + column count), by a counting sort over
+// bins: exact below 1,024, then 32 an octave (any order is a valid one).
+constexpr int kDegBins = 1024 + 22 * 32;
+
+__device__ __forceinline__ int degree_bin(const GatherList& gl, const int* __restrict__ colcnt, long long i) {
+  const long long d = gl.ptr[i + 1] - gl.ptr[i] + colcnt[i];
+  if (d < 1024) return (int)d;
+  const int x = (int)min(d, 0x7fffffffll), o = 31 - __clz(x);
+  return 1024 + (o - 10) * 32 + ((x >> (o - 5)) & 31);
+}
+
+__global__ void __launch_bounds__(1024) k_degree_hist(GatherList gl, const int* __restrict__ colcnt,
+                                                      int* __restrict__ hist) {
+  __shared__ int h[kDegBins];
+  for (int b = (int)threadIdx.x; b < kDegBins; b += 1024) h[b] = 0;
+  __syncthreads();
+  for (long long i = (long long)blockIdx.x * 1024 + threadIdx.x; i < gl.nrows; i += (long long)gridDim.x * 1024)
+    atomicAdd(h + degree_bin(gl, colcnt, i), 1);
+  __syncthreads();
+  for (int b = (int)threadIdx.x; b < kDegBins; b += 1024)
+    if (h[b]) atomicAdd(hist + b, h[b]);
+}
+
+// First rank of every bin, the highest degrees first (one block).
+__global__ void __launch_bounds__(1024) k_degree_starts(int* __restrict__ hist) {
+  __shared__ int warp_sh[32];
+  const unsigned lane = threadIdx.x & 31;
+  const int wib = (int)(threadIdx.x >> 5);
+  int carry = 0;
+  for (int b0 = 0; b0 < kDegBins; b0 += 1024) {
+    const int b = kDegBins - 1 - (b0 + (int)threadIdx.x);
+    const int c = b >= 0 ? hist[b] : 0;
+    int x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if ((int)lane >= o) x += y;
+    }
+    if (lane == 31) warp_sh[wib] = x;
+    __syncthreads();
+    int before = carry, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < wib) before += warp_sh[w];
+      all += warp_sh[w];
+    }
+    if (b >= 0) hist[b] = before + x - c;
+    carry += all;
+    __syncthreads();
+  }
+}
+
+// Ranks: a block counts its vertices per bin, reserves their places and deals
+// them out (few atomics reach one bin's counter).
+__global__ void __launch_bounds__(1024) k_degree_ranks(GatherList gl, const int* __restrict__ colcnt,
+                                                       int* __restrict__ next, int* __restrict__ rank) {
+  __shared__ int h[kDegBins], base[kDegBins];
+  constexpr int kPer = 4;
+  const long long i0 = (long long)blockIdx.x * 1024 * kPer;
+  for (int b = (int)threadIdx.x; b < kDegBins; b += 1024) h[b] = 0;
+  __syncthreads();
+  int bin[kPer], at[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const long long i = i0 + q * 1024 + threadIdx.x;
+    bin[q] = i < gl.nrows ? degree_bin(gl, colcnt, i) : -1;
+    at[q] = bin[q] >= 0 ? atomicAdd(h + bin[q], 1) : 0;
+  }
+  __syncthreads();
+  for (int b = (int)threadIdx.x; b < kDegBins; b += 1024)
+    if (h[b]) base[b] = atomicAdd(next + b, h[b]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (bin[q] >= 0) rank[i0 + q * 1024 + threadIdx.x] = base[bin[q]] + at[q];
+}
+
+// A warp per row of the lower triangle: count the edges of every owner -- the
+// end of higher rank -- (FILL = false), or put the other ends' ranks into the
+// owners' lists, in any order.
+template <bool FILL>
+__global__ void __launch_bounds__(kTPB) k_orient(GatherList gl, const int* __restrict__ rank, int* __restrict__ cnt,
+                                                 const long long* __restrict__ optr, int* __restrict__ ocol) {
+  constexpr int kPer = 4;  // entries of a lane in flight
+  const unsigned lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < gl.nrows; i += nwarps) {
+    const int ri = rank[i];
+    const long long e = gl.ptr[i + 1];
+    for (long long p = gl.ptr[i] + lane; p - lane < e; p += 32 * kPer) {
+      int rk[kPer], at[kPer];
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        rk[q] = p + 32 * q < e ? rank[gl.col[p + 32 * q]] : ri;
+        if (rk[q] != ri) at[q] = atomicAdd(cnt + max(ri, rk[q]), 1);  // the diagonal is left out
+      }
+#pragma unroll
+      for (int q = 0; q < kPer; ++q)
+        if (FILL && rk[q] != ri) ocol[optr[max(ri, rk[q])] + at[q]] = min(ri, rk[q]);
+    }
+  }
+}
+
+// A list of one entry has no pair in it.
+__global__ void k_tc_unit_counts(Lists l, int* __restrict__ cnt) {
+  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < l.n; u += (long long)gridDim.x * blockDim.x) {
+    const long long a = l.ptr[u + 1] - l.ptr[u];
+    cnt[u] = a < 2 ? 0 : (int)((a + kUnit - 1) / kUnit);
+  }
+}
+
+__global__ void k_tc_units(const int* __restrict__ unit0, int n, int* __restrict__ unit) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    for (int u = unit0[i]; u < unit0[i + 1]; ++u) unit[u] = (int)i;
+}
+
+__device__ __forceinline__ void add_count(unsigned long long acc, unsigned long long* count) {
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(count, acc);
+}
+
+// Rows of at most kShortRow entries and no diagonal, a lane each.
+__global__ void __launch_bounds__(kTPB) k_tc_lanes(GatherList gl, unsigned long long* __restrict__ count) {
+  unsigned long long acc = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < gl.nrows;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long p = gl.ptr[i];
+    const int a = (int)(gl.ptr[i + 1] - p);
+    int A[kShortRow];
+#pragma unroll
+    for (int q = 0; q < kShortRow; ++q) A[q] = q < a ? gl.col[p + q] : -1;
+#pragma unroll
+    for (int q = 1; q < kShortRow; ++q) {  // entry q's row holds entries before it only
+      if (q >= a) continue;
+      for (long long b = gl.ptr[A[q]], e = gl.ptr[A[q] + 1]; b < e; ++b) {
+        const int x = gl.col[b];
+#pragma unroll
+        for (int c = 0; c < q; ++c) acc += x == A[c];
+      }
+    }
+  }
+  add_count(acc, count);
+}
+
+__device__ __forceinline__ unsigned filter_bit(int c) { return ((unsigned)c * 2654435761u) >> 21; }  // of kFilterBits
+
+__global__ void __launch_bounds__(kTcWarps * 32) k_tc_warps(Lists l, const int* __restrict__ unit,
+                                                            const int* __restrict__ unit0, int nunits,
+                                                            unsigned long long* __restrict__ count) {
+  static_assert(kFilterBits == 2048, "filter_bit gives eleven bits");
+  __shared__ unsigned bits_sh[kTcWarps][kBits / 32];
+  __shared__ unsigned filter_sh[kTcWarps][kFilterBits / 32];
+  __shared__ int high_sh[kTcWarps][kPiece];  // the piece's ranks past the bitmap
+  const unsigned lane = threadIdx.x & 31;
+  const int wib = (int)(threadIdx.x >> 5);
+  unsigned *bits = bits_sh[wib], *filter = filter_sh[wib];
+  int* high = high_sh[wib];
+  for (int w = (int)lane; w < kBits / 32; w += 32) bits[w] = 0u;
+  for (int w = (int)lane; w < kFilterBits / 32; w += 32) filter[w] = 0u;
+  __syncwarp();
+  unsigned long long acc = 0;
+  const int nwarps = (int)gridDim.x * kTcWarps;
+  for (int q = (int)blockIdx.x * kTcWarps + wib; q < nunits; q += nwarps) {
+    const int u = unit[q];
+    const long long p = l.ptr[u];
+    const int a = (int)(l.ptr[u + 1] - p);
+    const int s = (q - unit0[u]) * kUnit, z = min(s + kUnit, a);  // the unit's entries
+    for (int h0 = 0; h0 < a; h0 += kPiece) {  // the list, in pieces
+      const int h1 = min(h0 + kPiece, a);
+      int nh = 0;
+      for (int c0 = h0; c0 < h1; c0 += 32) {
+        const int x = c0 + (int)lane < h1 ? l.col[p + c0 + lane] : -1;
+        const bool far = x >= kBits;
+        if (x >= 0 && !far) atomicOr(bits + (x >> 5), 1u << (x & 31));
+        if (far) atomicOr(filter + (filter_bit(x) >> 5), 1u << (filter_bit(x) & 31));
+        const unsigned m = __ballot_sync(0xffffffffu, far);
+        if (far) high[nh + __popc(m & ((1u << lane) - 1u))] = x;
+        nh += __popc(m);
+      }
+      __syncwarp();
+      for (int t0 = s; t0 < z; t0 += 32) {
+        long long bl = 0;
+        int nl = 0;
+        if (t0 + (int)lane < z) {
+          const int v = l.col[p + t0 + lane];
+          bl = l.ptr[v];
+          nl = (int)(l.ptr[v + 1] - bl);
+        }
+        const int m = min(32, z - t0);
+        unsigned hits = 0;
+        for (int j = 0; j < m; j += kSide) {
+          const int* B[kSide];
+          int nb[kSide], most = 0;
+#pragma unroll
+          for (int i = 0; i < kSide; ++i) {  // lanes from m on have nl = 0
+            B[i] = l.col + __shfl_sync(0xffffffffu, bl, (j + i) & 31);
+            nb[i] = __shfl_sync(0xffffffffu, nl, (j + i) & 31);
+            most = max(most, nb[i]);
+          }
+          for (int b = (int)lane; b < most; b += 32) {
+            int x[kSide];
+#pragma unroll
+            for (int i = 0; i < kSide; ++i) x[i] = b < nb[i] ? B[i][b] : -1;
+#pragma unroll
+            for (int i = 0; i < kSide; ++i) {
+              if ((unsigned)x[i] < (unsigned)kBits) {
+                hits += (bits[x[i] >> 5] >> (x[i] & 31)) & 1u;
+              } else if (nh > 0 && x[i] >= 0 && ((filter[filter_bit(x[i]) >> 5] >> (filter_bit(x[i]) & 31)) & 1u)) {
+                for (int c = 0; c < nh; ++c) hits += high[c] == x[i];
+              }
+            }
+          }
+        }
+        acc += hits;
+      }
+      __syncwarp();
+      for (int c = h0 + (int)lane; c < h1; c += 32) {  // leave both clear
+        const int x = l.col[p + c];
+        if (x < kBits) bits[x >> 5] = 0u;
+        else filter[filter_bit(x) >> 5] = 0u;
+      }
+      __syncwarp();
+    }
+  }
+  add_count(acc, count);
+}
+
+// The diagonal's share: for every entry (i, k) with i > k and k on the
+// diagonal 1 (k is common to rows i and k), for every diagonal (i, i) the
+// length of row i.
+__global__ void __launch_bounds__(kTPB) k_tc_diagonal(GatherList gl, unsigned long long* __restrict__ count) {
+  const unsigned lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  unsigned long long acc = 0;
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < gl.nrows; i += nwarps) {
+    const long long b = gl.ptr[i], e = gl.ptr[i + 1];
+    for (long long p = b + lane; p < e; p += 32) {
+      const int k = gl.col[p];
+      if (k == i) acc += (unsigned long long)(e - b);
+      else acc += gl.ptr[k + 1] > gl.ptr[k] && gl.col[gl.ptr[k + 1] - 1] == k;
+    }
+  }
+  add_count(acc, count);
 }
 
 // Block row of every tile (computed once per graph, from the work items).
@@ -312,9 +596,115 @@ __global__ void __launch_bounds__(kTPB) k_tc32_mma(GView v, long long nblk, cons
 
 }  // namespace
 
+namespace {
+
+// The lists and units of a lower triangle, once per graph.
+int build_lists(gbo_graph* g, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(g->build_mu);
+  if (g->tc_nunits >= 0) return GBO_OK;
+  const GatherList gl = gather_of(g);
+  const size_t n = (size_t)g->nrows;
+  const unsigned grid = std::min(blocks_for(g->nrows, 256), (unsigned)num_sms() * 8u);
+  const unsigned gw = std::min(blocks_for_warps(g->nrows, kTPB / 32), (unsigned)num_sms() * 8u);
+  char* tmp = nullptr;  // {total, bins, ranks, owners' counts, column counts}
+  GBO_CUDA_TRY(pool_malloc_async(&tmp, sizeof(long long) + sizeof(int) * (kDegBins + 3 * n), s));
+  const int st = [&]() -> int {
+    auto* tot = reinterpret_cast<long long*>(tmp);
+    int* bins = reinterpret_cast<int*>(tot + 1);
+    int *rank = bins + kDegBins, *own = rank + n;
+    const int* colcnt = g->outdeg;
+    if (!colcnt) {
+      int* c = own + n;
+      GBO_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(int) * n, s));
+      if (gl.nnz > 0)
+        k_count_cols<<<(unsigned)std::min<long long>((gl.nnz + 255) / 256, num_sms() * 32ll), 256, 0, s>>>(gl.col, gl.nnz, c);
+      colcnt = c;
+    }
+    GBO_TRY(list_alloc(&g->tc_ptr, n + 1, s));
+    GBO_TRY(list_alloc(&g->tc_col, (size_t)gl.nnz, s));
+    GBO_TRY(list_alloc(&g->tc_unit0, n + 1, s));
+    GBO_CUDA_TRY(cudaMemsetAsync(bins, 0, sizeof(int) * kDegBins, s));
+    k_degree_hist<<<std::min(blocks_for(g->nrows, 4096), (unsigned)num_sms() * 2u), 1024, 0, s>>>(gl, colcnt, bins);
+    k_degree_starts<<<1, 1024, 0, s>>>(bins);
+    k_degree_ranks<<<blocks_for(g->nrows, 4096), 1024, 0, s>>>(gl, colcnt, bins, rank);
+    GBO_CUDA_TRY(cudaMemsetAsync(own, 0, sizeof(int) * n, s));
+    k_orient<false><<<gw, kTPB, 0, s>>>(gl, rank, own, nullptr, nullptr);
+    GBO_TRY(exclusive_scan_i32_to_i64(own, g->tc_ptr, g->nrows, tot, s));
+    GBO_CUDA_TRY(cudaMemsetAsync(own, 0, sizeof(int) * n, s));
+    k_orient<true><<<gw, kTPB, 0, s>>>(gl, rank, own, g->tc_ptr, g->tc_col);
+    const Lists l{g->tc_ptr, g->tc_col, g->nrows};
+    k_tc_unit_counts<<<grid, 256, 0, s>>>(l, own);
+    GBO_TRY(exclusive_scan_i32(own, g->tc_unit0, g->nrows, tot, s));
+    long long nu = 0;
+    const cudaError_t e = read_back(&nu, tot, sizeof(nu), s);
+    if (e != cudaSuccess) return fail_cuda(e, "triangle count units");
+    if (nu > 2147483647ll) return fail(GBO_ERR_OVERFLOW, "triangle counting: too many entries");
+    GBO_TRY(list_alloc(&g->tc_unit, (size_t)nu, s));
+    if (nu > 0) k_tc_units<<<grid, 256, 0, s>>>(g->tc_unit0, g->nrows, g->tc_unit);
+    GBO_CUDA_TRY(cudaGetLastError());
+    GBO_CUDA_TRY(cudaStreamSynchronize(s));
+    g->device_bytes += 12LL * (g->nrows + 1) + 4LL * (gl.nnz + nu);
+    g->tc_nunits = (int)nu;
+    return GBO_OK;
+  }();
+  cudaFreeAsync(tmp, s);
+  if (st != GBO_OK) {  // nothing half-built stays
+    cudaStreamSynchronize(s);
+    cudaFree(g->tc_ptr);
+    cudaFree(g->tc_col);
+    cudaFree(g->tc_unit);
+    cudaFree(g->tc_unit0);
+    g->tc_ptr = nullptr;
+    g->tc_col = g->tc_unit = g->tc_unit0 = nullptr;
+  }
+  return st;
+}
+
+bool counted_by_lane(const gbo_graph* g) { return g->gl_short && !g->gl_diag; }
+
+// Whether the count goes over lists, which are built if need be.
+bool lists_ready(gbo_graph* g, cudaStream_t s, int* st) {
+  if (g->tc_mma || g->nblk < kListTiles) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cap);
+  const bool may_build = cap == cudaStreamCaptureStatusNone;
+  if (g->gl_nparts < 0 && !may_build) return false;
+  *st = build_gather(g, s);
+  if (*st == GBO_OK && !g->gl_lower) return false;
+  if (*st == GBO_OK && !counted_by_lane(g)) {
+    if (g->tc_nunits < 0 && !may_build) return false;
+    *st = build_lists(g, s);
+  }
+  if (*st == GBO_ERR_NOMEM) {
+    clear_error();
+    *st = GBO_OK;
+    return false;
+  }
+  return *st == GBO_OK;
+}
+
+}  // namespace
+
 int tc_launch(gbo_graph* g, unsigned long long* d_count, cudaStream_t s) {
   GBO_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s));
   if (g->nblk == 0) return GBO_OK;
+  int st = GBO_OK;
+  if (lists_ready(g, s, &st)) {
+    const unsigned cap = (unsigned)num_sms() * 4u;
+    if (counted_by_lane(g)) {
+      k_tc_lanes<<<std::min(blocks_for(g->nrows, kTPB), cap * 2), kTPB, 0, s>>>(gather_of(g), d_count);
+    } else {
+      const Lists l{g->tc_ptr, g->tc_col, g->nrows};
+      if (g->tc_nunits > 0)
+        k_tc_warps<<<std::min(blocks_for_warps(g->tc_nunits, kTcWarps), cap), kTcWarps * 32, 0, s>>>(
+            l, g->tc_unit, g->tc_unit0, g->tc_nunits, d_count);
+      if (g->gl_diag)
+        k_tc_diagonal<<<std::min(blocks_for_warps(g->nrows, kTPB / 32), cap * 2), kTPB, 0, s>>>(gather_of(g), d_count);
+    }
+    GBO_CUDA_TRY(cudaGetLastError());
+    return GBO_OK;
+  }
+  GBO_TRY(st);
   GView v = view_of(g);
   if (!g->tile_row) {  // block row of every tile, kept with the graph
     GBO_CUDA_TRY(cudaMalloc(&g->tile_row, sizeof(int) * (size_t)g->nblk));
@@ -370,8 +760,7 @@ extern "C" int gbo_tc(const gbo_graph* lower, uint64_t* h_count, gbo_stream_t st
   int st = tc_launch(const_cast<gbo_graph*>(lower), d, s);
   unsigned long long h = 0;
   if (st == GBO_OK) {
-    cudaError_t e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t e = read_back(&h, d, sizeof(h), s);
     if (e != cudaSuccess) st = fail_cuda(e, "tc readback");
   }
   cudaFreeAsync(d, s);
