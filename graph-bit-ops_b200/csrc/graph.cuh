@@ -84,7 +84,7 @@ struct gbo_graph {
   bool tc_mma = false;     // GBO_FLAG_TC_MMA: dense 32x32 mask tiles on the 1-bit MMA
   bool owns_outdeg = true;
   // balanced schedule
-  int chunk = 0;
+  int longest = 0;  // tiles of the longest block row
   int nitems = 0;
   gbo_item* items = nullptr;
   int nsplit = 0;
@@ -101,15 +101,9 @@ struct gbo_graph {
 
 namespace gbo {
 
-// Chunk (tiles per work item) for a tile width.
-inline int chunk_for(int b) {
-  switch (b) {
-    case 4: return 2048;
-    case 8: return 1024;
-    case 16: return 512;
-    case 32: return 256;
-    default: return 128;
-  }
+// Most tiles per work item for a tile width.
+__host__ __device__ constexpr int chunk_for(int b) {
+  return 8192 / b;
 }
 
 // Work items processed per warp: 32/b groups for b <= 32, one for b = 64.

@@ -754,11 +754,35 @@ __global__ void k_inv(const int* __restrict__ deg, int n, float* __restrict__ in
 }
 
 // ------------------------------------------------------------- schedule
-__global__ void k_sched_counts(const int* __restrict__ rowptr, int nbr, int chunk,
+// Tiles of the longest block row (*longest starts at 0).
+__global__ void k_sched_longest(const int* __restrict__ rowptr, int nbr, int* __restrict__ longest) {
+  int most = 0;
+  for (long long R = (long long)blockIdx.x * blockDim.x + threadIdx.x; R < nbr; R += (long long)gridDim.x * blockDim.x)
+    most = max(most, rowptr[R + 1] - rowptr[R]);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(longest, most);
+}
+
+// Tiles per work item.  A graph of many tiles takes `most` (chunk_for).  One
+// whose tiles do not give every SM 32 warps of such items, and whose longest
+// block row would run far past the others, is cut finer (`fine`): that row's
+// item set the time of every product (R-MAT of 20,001 rows, us: fp32 b = 8
+// 389 -> 34, b = 32 186 -> 54, Boolean b = 8 61 -> 12; counts at 25,001 rows,
+// b = 64, 29 -> 12; min-select at 120,001 rows, b = 16, 287 -> 140).  Without
+// such a row the split rows' second launch costs more than it gives (counts,
+// uniform of 100,003 rows, b = 8: 6.2 -> 12.3).
+struct Chunk {
+  int fine, most;
+  const int* longest;
+  __device__ __forceinline__ int tiles() const { return *longest > 4 * fine ? fine : most; }
+};
+
+__global__ void k_sched_counts(const int* __restrict__ rowptr, int nbr, Chunk by,
                                int* __restrict__ nchunk, int* __restrict__ nslot,
                                int* __restrict__ issplit) {
   long long R = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (R >= nbr) return;
+  const int chunk = by.tiles();
   int len = rowptr[R + 1] - rowptr[R];
   int k = len <= chunk ? 1 : (len + chunk - 1) / chunk;
   nchunk[R] = k;
@@ -766,12 +790,13 @@ __global__ void k_sched_counts(const int* __restrict__ rowptr, int nbr, int chun
   issplit[R] = k > 1 ? 1 : 0;
 }
 
-__global__ void k_sched_fill(const int* __restrict__ rowptr, int nbr, int chunk,
+__global__ void k_sched_fill(const int* __restrict__ rowptr, int nbr, Chunk by,
                              const int* __restrict__ item_off, const int* __restrict__ slot_off,
                              const int* __restrict__ split_off, gbo_item* __restrict__ items,
                              gbo_split* __restrict__ splits) {
   long long R = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (R >= nbr) return;
+  const int chunk = by.tiles();
   int t0 = rowptr[R], t1 = rowptr[R + 1];
   int len = t1 - t0;
   int k = len <= chunk ? 1 : (len + chunk - 1) / chunk;
@@ -1049,7 +1074,6 @@ int upload_outdeg(gbo_graph* g, const int* h_deg, int n, cudaStream_t s) {
 
 int build_schedule(gbo_graph* g, cudaStream_t s) {
   const int nbr = g->nbr;
-  g->chunk = chunk_for(g->b);
   if (nbr == 0) {
     g->nitems = 0;
     g->nsplit = 0;
@@ -1066,22 +1090,27 @@ int build_schedule(gbo_graph* g, cudaStream_t s) {
   item_off = issplit + n1;
   slot_off = item_off + n1;
   split_off = slot_off + n1;
-  GBO_CUDA_TRY(pool_malloc_async(&tot, sizeof(long long) * 3, s));
-  k_sched_counts<<<blocks_for(nbr, 256), 256, 0, s>>>(g->rowptr, nbr, g->chunk, nchunk, nslot,
-                                                      issplit);
+  GBO_CUDA_TRY(pool_malloc_async(&tot, sizeof(long long) * 4, s));
+  int* longest = reinterpret_cast<int*>(tot + 3);
+  GBO_CUDA_TRY(cudaMemsetAsync(longest, 0, sizeof(long long), s));
+  const long long even = g->nblk / ((long long)num_sms() * 32 * groups_per_warp(g->b));
+  const int most = chunk_for(g->b);
+  const Chunk by{(int)std::min<long long>(most, even / 32 * 32 + 32), most, longest};
+  k_sched_longest<<<std::min(blocks_for(nbr, 1024), (unsigned)num_sms()), 1024, 0, s>>>(g->rowptr, nbr, longest);
+  k_sched_counts<<<blocks_for(nbr, 256), 256, 0, s>>>(g->rowptr, nbr, by, nchunk, nslot, issplit);
   GBO_TRY(exclusive_scan_i32(nchunk, item_off, nbr, tot + 0, s));
   GBO_TRY(exclusive_scan_i32(nslot, slot_off, nbr, tot + 1, s));
   GBO_TRY(exclusive_scan_i32(issplit, split_off, nbr, tot + 2, s));
-  long long h[3];
-  GBO_CUDA_TRY(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, s));
-  GBO_CUDA_TRY(cudaStreamSynchronize(s));
+  long long h[4];
+  GBO_CUDA_TRY(read_back(h, tot, sizeof(h), s));
+  g->longest = (int)h[3];
   g->nitems = (int)h[0];
   g->nslots = (int)h[1];
   g->nsplit = (int)h[2];
   GBO_CUDA_TRY(cudaMalloc(&g->items, sizeof(gbo_item) * (size_t)(g->nitems > 0 ? g->nitems : 1)));
   GBO_CUDA_TRY(cudaMalloc(&g->splits, sizeof(gbo_split) * (size_t)(g->nsplit > 0 ? g->nsplit : 1)));
   g->device_bytes += sizeof(gbo_item) * (long long)g->nitems + sizeof(gbo_split) * (long long)g->nsplit;
-  k_sched_fill<<<blocks_for(nbr, 256), 256, 0, s>>>(g->rowptr, nbr, g->chunk, item_off, slot_off,
+  k_sched_fill<<<blocks_for(nbr, 256), 256, 0, s>>>(g->rowptr, nbr, by, item_off, slot_off,
                                                     split_off, g->items, g->splits);
   GBO_CUDA_TRY(cudaGetLastError());
   cudaFreeAsync(nchunk, s);
