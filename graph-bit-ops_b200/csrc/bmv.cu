@@ -13,6 +13,8 @@
 // loads of one tile are contiguous) and combines it with the x segment of
 // the tile's block column.  Items that cover a chunk of a split row write
 // partial results to scratch; k_reduce_* combines them in slot order.
+#include <algorithm>
+
 #include "scan.cuh"
 
 namespace gbo {
@@ -342,12 +344,18 @@ __global__ void __launch_bounds__(kTPB) k_semiring(GView v, const typename SRT<S
   const gbo_item it = v.items[item];
   A acc0 = sr_identity<SR>(), acc1 = sr_identity<SR>();
   auto comb = [](A& a, A b) { sr_combine<SR>(a, b); };
+  FoldShared* sh = nullptr;
+  if constexpr (B == 32) {
+    __shared__ FoldShared fold_sh[kTPB / 32];
+    sh = fold_sh + (threadIdx.x >> 5);
+  }
   if (SR == SR_FLOAT && p.degptr)
-    fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r,
+    fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r, sh,
                         [&](long long j) { return (A)float_term_deg((const float*)x, p.degptr, j); },
                         comb, acc0, acc1);
   else
-    fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r, [&](long long j) { return sr_term<SR>(x, p.scale, j); },
+    fold_row_cols<B, 4>(v, it.t0, it.t1, v.item_wbase ? v.item_wbase[item] : 0ll, r, sh,
+                        [&](long long j) { return sr_term<SR>(x, p.scale, j); },
                         comb, acc0, acc1);
   if (it.slot >= 0) {
     scratch[(size_t)it.slot * B + r] = acc0;
@@ -474,6 +482,32 @@ int masked_impl(const GView& v, const void* x, const void* mask, void* out, void
   return GBO_OK;
 }
 
+// z[j] = x[j] * scale[j], the fp32 term of a set column j.
+__global__ void k_terms(const float* __restrict__ x, const float* __restrict__ scale, long long n,
+                        float* __restrict__ z) {
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x)
+    z[j] = x[j] * scale[j];
+}
+
+// Where columns are met several times each, the terms are laid out first and
+// a set bit takes one gather instead of two (R-MAT 20, b = 32: 503 -> 479 us;
+// R-MAT 18, b = 64: 601 -> 558); under 2^20 tiles the launch costs as much
+// (R-MAT of 20,001 rows, b = 8: 33 -> 37).  The buffer comes from the pool, which a stream under
+// capture does not take.  (Degrees are not read ahead: a row pointer need
+// only reach as far as the set columns.)
+float* float_terms(const GView& v, long long nblk, const float* x, const float* scale, cudaStream_t s) {
+  if (!scale || v.ncols <= 0 || nblk < std::max(4ll * v.ncols, 1ll << 20)) return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  float* z = nullptr;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+      pool_malloc_async(&z, sizeof(float) * (size_t)v.ncols, s) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  k_terms<<<std::min(blocks_for(v.ncols, 256), (unsigned)num_sms() * 8u), 256, 0, s>>>(x, scale, v.ncols, z);
+  return z;
+}
+
 template <int B, int SR>
 int semiring_impl(const GView& v, const void* x, void* y, SrParams p, void* scratch,
                   cudaStream_t s) {
@@ -584,8 +618,14 @@ int bmv_float(const gbo_graph* g, const float* x, float* y, float alpha, const f
               float add, void* scratch, cudaStream_t s, const int* degptr) {
   GView v = view_of(g);
   SrParams p{alpha, add, scale, degptr};
+  float* z = degptr ? nullptr : float_terms(v, g->nblk, x, scale, s);
+  if (z) {
+    x = z;
+    p.scale = nullptr;
+  }
   int st = GBO_OK;
   GBO_DISPATCH_B(g->b, st = (semiring_impl<B, SR_FLOAT>(v, x, y, p, scratch, s)));
+  if (z) cudaFreeAsync(z, s);
   return st;
 }
 

@@ -212,22 +212,52 @@ __device__ __forceinline__ unsigned warp_transpose32(unsigned x, unsigned lane) 
   return x;
 }
 
+// Position of the k-th set bit (from 0) of a word with more than k of them.
+__device__ __forceinline__ int nth_bit(unsigned x, int k) {
+  int at = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const int c = __popc((x >> at) & ((1u << s) - 1u));
+    if (k >= c) {
+      k -= c;
+      at += s;
+    }
+  }
+  return at;
+}
+
+constexpr int kThinWords = 6;
+
+// Shared memory of one warp's fold over b = 32 tiles with packed row words.
+struct FoldShared {
+  unsigned short slot[32 * kThinWords];  // a thin batch's words, row after row: tile of the batch | word << 5
+  uint2 row[32];              // first slot of every row, tiles of the batch where it is non-empty
+};
+
 // fold_row_cols (below) for b = 32 tiles with packed row words.  Per batch
 // of 32 tiles the occupancy words are transposed (lane r: the tiles where
-// row r is non-empty), and the batch's non-empty words are dealt out to the
-// lanes in row-major order, 32 per round: lane p takes word p (its row by a
-// binary search over the rows' prefix counts, its tile as the k-th tile of
-// that row), folds the word's columns (first set column, then the others in
-// order), and a segmented scan over the lanes of each row's run (the runs
-// are contiguous) leaves the run's fold in its last lane, which the row's
-// own lane folds into its accumulator.  Every lane does one word per round
-// whatever the rows' lengths (two rounds at a time, so that their loads
-// overlap), and the order of every fold is fixed by the graph alone.
-template <int U, typename Acc, typename Term, typename Comb>
-__device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1, long long wb,
-                                                  unsigned lane, Term term, Comb comb, Acc& acc) {
-  const unsigned* __restrict__ words = v.rowword;
+// row r is non-empty) and the non-empty words are dealt out to the lanes in
+// row-major order, 32 per round.  Where no tile has more than kThinWords of
+// them, the lane of every tile writes its words' places into shared memory;
+// else a lane finds its word (its row by a binary search over the rows'
+// prefix counts, its tile as the k-th tile of that row).  A lane folds its word's columns (first
+// set column, then the others in order), a segmented scan over the lanes of
+// each row's run (the runs are contiguous) leaves the run's fold in its last
+// lane, and the row's own lane folds that into its accumulator.  Every lane
+// does one word per round whatever the rows' lengths, and the order of every
+// fold is fixed by the graph alone.
+//
+// Bound by instructions (464 a batch with a search per word, 290 with places)
+// and then by the gathers' latency.  Searching with __fns in every batch /
+// this, us: fp32, uniform of 1,000,003 rows, 24 a row 426 / 312, of 20,001 rows
+// 22.5 / 12.3, R-MAT 20 545 / 479, mesh of 10^6 rows 43 / 39; min-plus, R-MAT 20
+// 432 / 413.  Places in all batches: R-MAT 20 569, mesh 51 (one tile with 32
+// words keeps 31 lanes waiting).
+template <typename Acc, typename Term, typename Comb>
+__device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1, long long wb, unsigned lane,
+                                                  FoldShared& sh, Term term, Comb comb, Acc& acc) {
   const unsigned* __restrict__ rm = v.rowmask;
+  const unsigned before = (1u << lane) - 1u;
   int cn = t0 + (int)lane < t1 ? v.colind[t0 + lane] : 0;
   unsigned mn = t0 + (int)lane < t1 ? rm[t0 + lane] : 0u;
   for (int b0 = t0; b0 < t1; b0 += 32) {
@@ -238,40 +268,27 @@ __device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1
       cn = t < t1 ? v.colind[t] : 0;
       mn = t < t1 ? rm[t] : 0u;
     }
+    const unsigned* __restrict__ words = v.rowword + wb;
     const int mc = __popc(m);
-    const int off = warp_incl_sum(mc, lane) - mc;  // lane j: tile j's first word, relative to wb
-    const long long wbat = wb;
     const unsigned tl = warp_transpose32(m, lane);  // lane r: tiles of the batch where row r is non-empty
     const int rc = __popc(tl);
-    const int rincl = warp_incl_sum(rc, lane);
+    // both prefix sums at once (at most 1,024 words)
+    const int both = warp_incl_sum(mc | rc << 16, lane);
+    const int off = (both & 0xffff) - mc;  // lane j: tile j's first word, relative to wb
+    const int rincl = both >> 16, rexcl = rincl - rc;
     const int total = __shfl_sync(0xffffffffu, rincl, 31);
     wb += total;
-    const int rexcl = rincl - rc;
-    constexpr int H = 2;  // rounds dealt together (their loads overlap)
-    for (int pb = 0; pb < total; pb += 32 * H) {
+    // 32 * H words dealt from word pb on; where(p): word p's tile | its index << 5
+    auto deal = [&](auto hc, int pb, auto where) {
+      constexpr int H = decltype(hc)::value;
       Acc x[H];
-      int key[H];
-      unsigned w[H];
-      long long base[H];
+      unsigned w[H], base[H];
 #pragma unroll
       for (int h = 0; h < H; ++h) {
         const int p = pb + 32 * h + (int)lane;
-        // row of word p: the number of rows whose inclusive count is <= p
-        int r = 0;
-#pragma unroll
-        for (int st = 16; st > 0; st >>= 1) {
-          const int c = __shfl_sync(0xffffffffu, rincl, r + st - 1);
-          if (c <= p) r += st;
-        }
-        const int er = __shfl_sync(0xffffffffu, rexcl, r);
-        const unsigned tr = __shfl_sync(0xffffffffu, tl, r);
-        const bool valid = p < total;
-        const int j = valid ? (int)__fns(tr, 0, p - er + 1) : 0;
-        const unsigned mj = __shfl_sync(0xffffffffu, m, j);
-        const int oj = __shfl_sync(0xffffffffu, off, j);
-        base[h] = (long long)__shfl_sync(0xffffffffu, cb, j) * 32;
-        w[h] = valid ? words[wbat + oj + __popc(mj & ((1u << r) - 1u))] : 0u;
-        key[h] = valid ? r : -1 - (int)lane;
+        const unsigned q = where(p);
+        base[h] = (unsigned)__shfl_sync(0xffffffffu, cb, (int)(q & 31u)) * 32u;  // < 2^32: ncols is an int
+        w[h] = p < total ? words[q >> 5] : 0u;
       }
       // the first set column of each word gathered together, then the others
 #pragma unroll
@@ -291,14 +308,17 @@ __device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1
           comb(x[h], term(base[h] + col));
         }
       }
-      // segmented inclusive scan over each row's run of lanes, per round
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
+      for (int h = 0; h < H; ++h) {
+        const int rb = pb + 32 * h;
+        // first lane of this lane's run: the last run that starts at or before it
+        const bool starts = rc > 0 && rexcl >= rb && rexcl < rb + 32;
+        const unsigned heads = __reduce_or_sync(0xffffffffu, starts ? 1u << (rexcl - rb) : 0u) | 1u;
+        const int first = 31 - __clz((int)(heads & (before << 1 | 1u)));
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
+        for (int d = 1; d < 32; d <<= 1) {
           const Acc y = __shfl_up_sync(0xffffffffu, x[h], d);
-          const int ky = __shfl_up_sync(0xffffffffu, key[h], d);
-          if ((int)lane >= d && ky == key[h]) {
+          if ((int)lane >= first + d) {
             Acc z = y;
             comb(z, x[h]);
             x[h] = z;
@@ -313,6 +333,34 @@ __device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1
         const Acc seg = __shfl_sync(0xffffffffu, x[h], hi > lo ? hi - 1 - rb : 0);
         if (hi > lo) comb(acc, seg);
       }
+    };
+    if (__reduce_max_sync(0xffffffffu, mc) <= kThinWords) {
+      sh.row[lane] = make_uint2((unsigned)rexcl, tl);
+      __syncwarp();
+      unsigned at = (unsigned)off << 5 | lane;
+      for (unsigned mm = m; mm; mm &= mm - 1, at += 32) {
+        const uint2 q = sh.row[__ffs(mm) - 1];
+        sh.slot[q.x + __popc(q.y & before)] = (unsigned short)at;
+      }
+      __syncwarp();
+      for (int pb = 0; pb < total; pb += 32)
+        deal(std::integral_constant<int, 1>{}, pb, [&](int p) { return p < total ? (unsigned)sh.slot[p] : 0u; });
+      __syncwarp();
+    } else {
+      for (int pb = 0; pb < total; pb += 64)
+        deal(std::integral_constant<int, 2>{}, pb, [&](int p) {
+          int r = 0;  // rows whose inclusive count is at most p
+#pragma unroll
+          for (int st = 16; st > 0; st >>= 1) {
+            const int c = __shfl_sync(0xffffffffu, rincl, r + st - 1);
+            if (c <= p) r += st;
+          }
+          const int er = __shfl_sync(0xffffffffu, rexcl, r);
+          const unsigned tr = __shfl_sync(0xffffffffu, tl, r);
+          const int j = p < total ? nth_bit(tr, p - er) : 0;
+          const unsigned mj = __shfl_sync(0xffffffffu, m, j);
+          return ((unsigned)__shfl_sync(0xffffffffu, off, j) + __popc(mj & ((1u << r) - 1u))) << 5 | (unsigned)j;
+        });
     }
   }
 }
@@ -330,14 +378,14 @@ __device__ __forceinline__ void fold_row_cols_t32(const GView& v, int t0, int t1
 // in 32 bits for b <= 32 (64 for b = 64) so that column 0 is the top bit.
 template <int B, int U, typename Acc, typename Term, typename Comb>
 __device__ __forceinline__ void fold_row_cols(const GView& v, int t0, int t1, long long wb, int r,
-                                              Term term, Comb comb, Acc& acc0, Acc& acc1) {
+                                              FoldShared* sh, Term term, Comb comb, Acc& acc0, Acc& acc1) {
   using WT = typename Word<B>::T;
   using L = Lay<B>;
   using T = decltype(term(0ll));
   using AW = typename std::conditional<(B > 32), unsigned long long, unsigned>::type;
   if constexpr (B == 32) {
     if (v.rowword) {
-      fold_row_cols_t32<U>(v, t0, t1, wb, (unsigned)r, term, comb, acc0);
+      fold_row_cols_t32(v, t0, t1, wb, (unsigned)r, *sh, term, comb, acc0);
       return;
     }
   }
