@@ -1764,7 +1764,8 @@ int finish_loop(AlgoState* a, cudaStream_t s, int max_iter, int cap_iters, int* 
   a->replays = 1;
   a->stats_pending = true;
   if (!iters && cap_iters == 0 && !must_wait) return GBO_OK;
-  GBO_CUDA_TRY(cudaMemcpyAsync(a->h_ctrl, a->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
+  // the loop's outcome, without the per-level counters behind it
+  GBO_CUDA_TRY(cudaMemcpyAsync(a->h_ctrl, a->ctrl, offsetof(Ctrl, err_part), cudaMemcpyDeviceToHost, s));
   GBO_CUDA_TRY(cudaStreamSynchronize(s));
   if (coop && a->h_ctrl->bar_err) return fail(GBO_ERR_TIMEOUT, "cooperative loop: a grid barrier gave up");
   if (!a->h_ctrl->done) return fail(GBO_ERR_TIMEOUT, "iteration loop did not terminate");
@@ -1788,7 +1789,10 @@ int run_until_done(AlgoState* a, int id, cudaStream_t s, int max_iter, int* iter
 // barrier needs it) and at most kCoopBlocksPerSM per SM -- a barrier costs
 // 2.4 us over 148 blocks and 4.0 us over 888 on B200, and R-MAT 22 BFS runs
 // fastest at 4-5 blocks per SM -- and about one warp per 4 block rows or 32
-// work items; or the caller's choice (gbo_graph_set_bfs_loop) within the
+// work items, but up to two blocks an SM one per block row: a level of a small
+// graph takes as long as its busiest warp (us at a quarter of the warps / now:
+// uniform of 1,000 rows 56 / 42, of 4,000 59 / 43, mesh of 2,025 290 / 218,
+// uniform of 100,000 72 / 67); or the caller's choice (gbo_graph_set_bfs_loop) within the
 // resident limit.
 int coop_grid(const gbo_graph* g, unsigned* grid) {
   int per_sm = 0, coop = 0, dev = 0;
@@ -1800,6 +1804,8 @@ int coop_grid(const gbo_graph* g, unsigned* grid) {
   const unsigned cap = (unsigned)num_sms() * (unsigned)per_sm;
   const long long warps = std::max<long long>(((long long)g->nbr + 3) / 4, ((long long)g->nitems + 31) / 32);
   unsigned want = blocks_for_warps(std::max<long long>(warps, 1), kTPB / 32);
+  // up to two blocks an SM, a warp per block row
+  want = std::max(want, std::min(blocks_for_warps(std::max(g->nbr, 1), kTPB / 32), (unsigned)num_sms() * 2u));
   want = std::min(want, (unsigned)num_sms() * (unsigned)kCoopBlocksPerSM);
   if (g->bfs_coop_blocks > 0) want = (unsigned)g->bfs_coop_blocks;
   *grid = want < cap ? want : cap;
@@ -1894,13 +1900,14 @@ int bfs_impl(gbo_graph* g, int src, const int* h_seeds, int nseeds, int32_t* d_l
   // the slice pull step finishes every block row itself: no split partials
   GView vfin = v;
   if (rws) vfin.nsplit = 0;
-  const unsigned gi = col ? grid_persistent(k_bfs_step_col<B>, g->nitems)
+  const unsigned gi = coop ? 0u
+                      : col ? grid_persistent(k_bfs_step_col<B>, g->nitems)
                           : rws ? grid_persistent(k_bfs_pull_rws, ((long long)g->nbr + 31) / 32)
                                 : grid_items_persistent(k_bfs_step<B>, g->nitems, B);
   // push steps (symmetric graphs) finalise every block row in k_bfs_finish
   const bool push_ok = g->symmetric;
   const unsigned gs = blocks_for(std::max<long long>(g->nsplit, push_ok ? g->nbr : 0), kTPB);
-  const unsigned gp = col ? grid_persistent(k_bfs_push_col<B>, g->nitems) : grid_persistent(k_bfs_push<B>, g->nitems);
+  const unsigned gp = coop ? 0u : col ? grid_persistent(k_bfs_push_col<B>, g->nitems) : grid_persistent(k_bfs_push<B>, g->nitems);
   if (!coop) GBO_TRY(get_exec(a, A_BFS, nullptr, [&](cudaStream_t cs, int k, int* nl) -> int {
     if (g->nitems > 0) {
       if (col) k_bfs_step_col<B><<<gi, kTPB, 0, cs>>>(v, front, vis, level, ctrl, scratch);
