@@ -133,15 +133,15 @@ __device__ __forceinline__ void tile_counts(const void* __restrict__ val, long l
   }
 }
 
-template <int B, bool OUTF>
+template <int B, bool OUTF, bool WHOLE>
 __global__ void __launch_bounds__(kTPB) k_count_narrow(GView v, const typename Word<B>::T* __restrict__ x,
                                                        void* __restrict__ yv, int accumulate,
-                                                       int* __restrict__ scratch, bool whole) {
+                                                       int* __restrict__ scratch) {
   const unsigned lane = threadIdx.x & 31;
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (item >= v.nitems) return;
   gbo_item it = v.items[item];
-  if (whole && it.slot >= 0) {  // the first item takes the row
+  if (WHOLE && it.slot >= 0) {  // the first item takes the row
     const int r0 = v.rowptr[it.row];
     if (it.t0 != r0) return;
     it = gbo_item{it.row, r0, v.rowptr[it.row + 1], -1};
@@ -444,10 +444,14 @@ int count_impl(const GView& v, int longest, const void* x, void* y, int out_type
       narrow = (reinterpret_cast<uintptr_t>(v.val) % kAlign) == 0;
       if (narrow) {
         const unsigned grid = blocks_for_warps(v.nitems, kTPB / 32);
-        if (out_type == GBO_OUT_F32)
-          k_count_narrow<B, true><<<grid, kTPB, 0, s>>>(v, (const WT*)x, y, accumulate, scratch, whole);
-        else
-          k_count_narrow<B, false><<<grid, kTPB, 0, s>>>(v, (const WT*)x, y, accumulate, scratch, whole);
+        auto run = [&](auto f32, auto rows) {
+          k_count_narrow<B, decltype(f32)::value, decltype(rows)::value>
+              <<<grid, kTPB, 0, s>>>(v, (const WT*)x, y, accumulate, scratch);
+        };
+        const std::true_type yes;
+        const std::false_type no;
+        if (out_type == GBO_OUT_F32) whole ? run(yes, yes) : run(yes, no);
+        else whole ? run(no, yes) : run(no, no);
       }
     }
     if (!narrow) {
