@@ -362,7 +362,10 @@ GBO_API int gbo_cc(const gbo_graph* g, int32_t* d_label, int* h_iters,
  * (L L^T)[i][k].  Replaces tril_csr + bmm*_sparse_masked_v5 with a uint64
  * result (bsrbmm/bsrbmm.cu:1214-1265, 1416; bsrbmm/tc.cu:767-951). */
 GBO_API int gbo_tc(const gbo_graph* lower, uint64_t* h_count, gbo_stream_t stream);
-/* Same, result left in device memory (*d_count is overwritten). */
+/* Same, result left in device memory (*d_count is overwritten).  Returns once
+ * queued, except that the first count on a graph of 65,536 tiles or more builds
+ * the graph's neighbour lists and waits for the stream (under stream capture it
+ * counts over the tiles instead). */
 GBO_API int gbo_tc_device(const gbo_graph* lower, unsigned long long* d_count,
                   gbo_stream_t stream);
 
