@@ -381,20 +381,22 @@ __global__ void __launch_bounds__(kWideTPB) k_pack_wide(const int* __restrict__ 
       if (un.index > 0) wa = min((long long)max(colind[b0 + len * un.index / un.count], 0) / B, (long long)nbc);
       if (un.index + 1 < un.count)
         wz = min((long long)max(colind[b0 + len * (un.index + 1) / un.count], 0) / B, (long long)nbc);
-      if (!BUILD) {
-        // this unit's share of the slab's entries checked one by one (the
-        // rows' searches below suppose them sorted)
-        const int e0 = rp[0];
-        const long long ne = rp[rows] - e0;
-        const long long ez = e0 + ne * (un.index + 1) / un.count;
-        for (long long e = e0 + ne * un.index / un.count + tid; e < ez; e += kWideTPB) {
-          const int c = colind[e];
-          if (c < 0 || c >= ncols) atomicOr(derr, DERR_COL_BOUNDS);
-          if (e > e0 && c < colind[e - 1]) {
-            bool starts = false;
-            for (int r = 0; r < rows; ++r) starts = starts || rp[r] == (int)e;
-            if (!starts) atomicOr(derr, DERR_UNSORTED);
-          }
+    }
+    // The rows' searches below suppose sorted rows and leave out what lies past
+    // the last block column: where they are made, this unit's share of the
+    // slab's entries is checked one by one (a hub's units before the fill
+    // pass, by the count form).
+    if (un.count > 1 ? !BUILD : win < nbc) {
+      const int e0 = rp[0];
+      const long long ne = rp[rows] - e0;
+      const long long ez = e0 + ne * (un.index + 1) / un.count;
+      for (long long e = e0 + ne * un.index / un.count + tid; e < ez; e += kWideTPB) {
+        const int c = colind[e];
+        if (c < 0 || c >= ncols) atomicOr(derr, DERR_COL_BOUNDS);
+        if (e > e0 && c < colind[e - 1]) {
+          bool starts = false;
+          for (int r = 0; r < rows; ++r) starts = starts || rp[r] == (int)e;
+          if (!starts) atomicOr(derr, DERR_UNSORTED);
         }
       }
     }

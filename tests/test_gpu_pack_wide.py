@@ -88,3 +88,30 @@ def test_errors_inside_a_wide_slab(gbo, gpu, b):
     with pytest.raises(gbo.GboError) as e:
         _pack(gbo, ptr, col, b, ncols, b, 0)
     assert e.value.status == gbo.GBO_ERR_BOUNDS
+
+
+@pytest.mark.parametrize("nbc", [1_000_003, 2_100_000])
+@pytest.mark.parametrize("b", [4, 16, 32, 64])
+def test_errors_past_one_window(gbo, gpu, b, nbc):
+    """Bad entries that no window's search returns: columns below the first and
+    past the last block column, and (three windows) a stretch of a row moved so
+    that the end of one window and the start of the next lie apart."""
+    ncols = nbc * b - 3
+    n = min(400, 4000 // b)  # a slab of one unit
+    row = np.arange(n, dtype=np.int64) * ncols // n
+    good = [row + i for i in range(b)]
+    a, m = n // 20, n - n // 10
+    bads = [(np.concatenate([row[a:m], row[:a], row[m:]]), gbo.GBO_ERR_UNSORTED),
+            (np.concatenate([[-1], row]), gbo.GBO_ERR_BOUNDS),
+            (np.concatenate([[-9 * b], row]), gbo.GBO_ERR_BOUNDS),
+            (np.concatenate([row, [ncols]]), gbo.GBO_ERR_BOUNDS),
+            (np.concatenate([row, [ncols + 3 + b]]), gbo.GBO_ERR_BOUNDS)]
+    for bad, status in bads:
+        rows = list(good)
+        rows[b // 2] = bad
+        ptr, col = _csr(rows, ncols)
+        with pytest.raises(gbo.GboError) as e:
+            _pack(gbo, ptr, col, b, ncols, b, 0)
+        assert e.value.status == status
+    ptr, col = _csr(good, ncols)
+    _pack(gbo, ptr, col, b, ncols, b, 0)
