@@ -108,8 +108,8 @@ void destroy(gbo_graph* g) {
   }
   if (g->owns_outdeg) cudaFree(g->outdeg);
   cudaFree(g->perm);
+  lists_idle(g->tile_row ? static_cast<void*>(g->tile_row) : g->tc_ptr);
   cudaFree(g->tile_row);
-  lists_idle(g->tc_ptr);
   cudaFree(g->tc_ptr);
   cudaFree(g->tc_col);
   cudaFree(g->tc_unit);

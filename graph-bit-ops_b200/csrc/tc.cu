@@ -31,8 +31,9 @@
 // kListTiles are counted in about 100 (uniform of 10,000 vertices, 65,764
 // tiles: 90, with lists 42, the first call 240; R-MAT of 20,001, 122,369:
 // 347, 54, 410).  Fewer tiles, tensor-core counts and matrices with an entry
-// above the diagonal keep the tile kernels, as does a first call under stream
-// capture, where nothing can be read back, or without memory for the lists.
+// above the diagonal keep the tile kernels, as does a call under stream capture
+// before the lists are built (nothing can be read back there) or one without
+// memory for them.
 #include <algorithm>
 
 #include "gather.cuh"
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kTPB) k_tc_diagonal(GatherList gl, unsigned lo
   add_count(acc, count);
 }
 
-// Block row of every tile (computed once per graph, from the work items).
+// Block row of every tile, from the work items.
 __global__ void k_tile_row(GView v, int* __restrict__ tile_row) {
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (item >= v.nitems) return;
@@ -662,12 +663,15 @@ int build_lists(gbo_graph* g, cudaStream_t s) {
 
 bool counted_by_lane(const gbo_graph* g) { return g->gl_short && !g->gl_diag; }
 
-// Whether the count goes over lists, which are built if need be.
-bool lists_ready(gbo_graph* g, cudaStream_t s, int* st) {
-  if (g->tc_mma || g->nblk < kListTiles) return false;
+bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(s, &cap);
-  const bool may_build = cap == cudaStreamCaptureStatusNone;
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Whether the count goes over lists, which are built if need be.
+bool lists_ready(gbo_graph* g, cudaStream_t s, bool may_build, int* st) {
+  if (g->tc_mma || g->nblk < kListTiles) return false;
   if (g->gl_nparts < 0 && !may_build) return false;
   *st = build_gather(g, s);
   if (*st == GBO_OK && !g->gl_lower) return false;
@@ -683,13 +687,41 @@ bool lists_ready(gbo_graph* g, cudaStream_t s, int* st) {
   return *st == GBO_OK;
 }
 
+// The tiles' block rows: made by the first direct count, complete when it goes
+// on (any stream may read them then), and kept with the graph.  A count under
+// capture before that queues an array of its own (`own`, freed in stream order:
+// nodes of the captured graph), since nothing it records has run yet.
+int tile_rows(gbo_graph* g, cudaStream_t s, bool may_build, int** rows, bool* own) {
+  std::lock_guard<std::mutex> lk(g->build_mu);
+  *own = false;
+  *rows = g->tile_row;
+  if (*rows) return GBO_OK;
+  int* t = nullptr;
+  GBO_TRY(list_alloc(&t, (size_t)g->nblk, s));
+  k_tile_row<<<blocks_for_warps(g->nitems, kTPB / 32), kTPB, 0, s>>>(view_of(g), t);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && may_build) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(t, s);
+    return fail_cuda(e, "tiles' block rows");
+  }
+  *rows = t;
+  *own = !may_build;
+  if (may_build) {
+    g->tile_row = t;
+    g->device_bytes += 4LL * g->nblk;
+  }
+  return GBO_OK;
+}
+
 }  // namespace
 
 int tc_launch(gbo_graph* g, unsigned long long* d_count, cudaStream_t s) {
   GBO_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s));
   if (g->nblk == 0) return GBO_OK;
   int st = GBO_OK;
-  if (lists_ready(g, s, &st)) {
+  const bool may_build = !capturing(s);
+  if (lists_ready(g, s, may_build, &st)) {
     const unsigned cap = (unsigned)num_sms() * 4u;
     if (counted_by_lane(g)) {
       k_tc_lanes<<<std::min(blocks_for(g->nrows, kTPB), cap * 2), kTPB, 0, s>>>(gather_of(g), d_count);
@@ -706,28 +738,28 @@ int tc_launch(gbo_graph* g, unsigned long long* d_count, cudaStream_t s) {
   }
   GBO_TRY(st);
   GView v = view_of(g);
-  if (!g->tile_row) {  // block row of every tile, kept with the graph
-    GBO_CUDA_TRY(cudaMalloc(&g->tile_row, sizeof(int) * (size_t)g->nblk));
-    g->device_bytes += 4LL * g->nblk;
-    k_tile_row<<<blocks_for_warps(g->nitems, kTPB / 32), kTPB, 0, s>>>(v, g->tile_row);
-  }
+  int* rows = nullptr;
+  bool own = false;
+  GBO_TRY(tile_rows(g, s, may_build, &rows, &own));
   long long warps = g->nblk;
   long long cap = (long long)num_sms() * 64;  // 64 resident warps per SM
   if (warps > cap * 8) warps = cap * 8;
   const unsigned grid = blocks_for_warps(warps, kTPB / 32);
   switch (g->b) {
-    case 4: k_tc<4><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 0, d_count); break;
-    case 8: k_tc<8><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 0, d_count); break;
-    case 16: k_tc<16><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 0, d_count); break;
+    case 4: k_tc<4><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 0, d_count); break;
+    case 8: k_tc<8><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 0, d_count); break;
+    case 16: k_tc<16><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 0, d_count); break;
     case 32: if (g->tc_mma) {
-      k_tc<32><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 1, d_count);
-      k_tc32_mma<<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, d_count);
+      k_tc<32><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 1, d_count);
+      k_tc32_mma<<<grid, kTPB, 0, s>>>(v, g->nblk, rows, d_count);
     } else {
-      k_tc<32><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 0, d_count);
+      k_tc<32><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 0, d_count);
     }; break;
-    default: k_tc<64><<<grid, kTPB, 0, s>>>(v, g->nblk, g->tile_row, 0, d_count); break;
+    default: k_tc<64><<<grid, kTPB, 0, s>>>(v, g->nblk, rows, 0, d_count); break;
   }
-  GBO_CUDA_TRY(cudaGetLastError());
+  const cudaError_t e = cudaGetLastError();
+  if (own) cudaFreeAsync(rows, s);
+  if (e != cudaSuccess) return fail_cuda(e, "triangle count");
   return GBO_OK;
 }
 
