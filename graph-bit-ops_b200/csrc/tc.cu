@@ -73,11 +73,13 @@ __global__ void k_count_cols(const int* __restrict__ col, long long nnz, int* __
 }
 
 // Ranks by falling degree (row length + column count), by a counting sort over
-// bins: exact below 1,024, then 32 an octave (any order is a valid one).
+// bins: exact below 1,024, then 32 an octave (any order is a valid one, so the
+// out-degrees that came with a wrapped graph need not be right: they are held
+// within the bins).
 constexpr int kDegBins = 1024 + 22 * 32;
 
 __device__ __forceinline__ int degree_bin(const GatherList& gl, const int* __restrict__ colcnt, long long i) {
-  const long long d = gl.ptr[i + 1] - gl.ptr[i] + colcnt[i];
+  const long long d = max(gl.ptr[i + 1] - gl.ptr[i] + colcnt[i], 0ll);
   if (d < 1024) return (int)d;
   const int x = (int)min(d, 0x7fffffffll), o = 31 - __clz(x);
   return 1024 + (o - 10) * 32 + ((x >> (o - 5)) & 31);

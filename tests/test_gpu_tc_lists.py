@@ -74,3 +74,20 @@ def test_entry_above_the_diagonal(gbo, orc, gpu, b):
     g = gbo.Graph.from_csr(gbo.Csr(rowptr, colind, n, n), b)
     assert g.info().nblocks >= TILES
     assert g.tc() == orc.tc_b2sr(orc.pack(rowptr, colind, n, n, b))
+
+
+@pytest.mark.parametrize("b", [8, 32])
+def test_wrapped_graph_with_wrong_degrees(gbo, orc, gpu, b):
+    """The out-degrees of a wrapped graph order the lists and no more: any
+    numbers give the same count."""
+    n = 36_001
+    rowptr, colind = _lower(gbo, "dense", n, False)
+    want = orc.tc_b2sr(orc.pack(rowptr, colind, n, n, b))
+    rp, ci, words = gbo.Graph.from_csr(gbo.Csr(rowptr, colind, n, n), b).b2sr()
+    rng = np.random.default_rng(b)
+    deg = rng.choice(np.array([-2**31, -70_000, -1, 0, 1, 1023, 1024, 2**31 - 1]), n).astype(np.int32)
+    bufs = [gbo.DeviceBuffer.from_numpy(a) for a in (rp, ci, words, deg)]
+    g = gbo.Graph.wrap_b2sr(n, n, b, 0, len(ci), *bufs)
+    assert g.info().nblocks >= TILES
+    for _ in range(2):
+        assert g.tc() == want
