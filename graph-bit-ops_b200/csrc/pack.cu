@@ -1276,42 +1276,69 @@ __global__ void k_rws_fill(const int* __restrict__ rowptr, const int* __restrict
   }
 }
 
-int build_rws(gbo_graph* g, cudaStream_t s) {
-  if (g->b != 32 || g->layout != GBO_LAYOUT_ROW || !g->rowmask || g->rws_head || g->nbr <= 0) return GBO_OK;
+namespace {
+
+// The slices while they are built: they become the graph's when complete.
+struct Slices {
+  uint2 *head = nullptr, *tail = nullptr;
+  long long *tail_ptr = nullptr, *long_chunk0 = nullptr, *chunk_beg = nullptr, *chunk_end = nullptr;
+  int *long_row = nullptr, *chunk_row = nullptr;
+  unsigned* longbits = nullptr;
+  long long ntail = 0, nchunk = 0, bytes = 0;
+  int nlong = 0;
+
+  template <typename T>
+  int make(T** p, size_t count) {
+    const size_t nb = sizeof(T) * (count > 0 ? count : 1);
+    GBO_CUDA_TRY(cudaMalloc(p, nb));
+    bytes += (long long)nb;
+    return GBO_OK;
+  }
+  template <typename T>
+  int upload(T** p, const std::vector<T>& src) {
+    GBO_TRY(make(p, src.size()));
+    if (!src.empty()) GBO_CUDA_TRY(cudaMemcpy(*p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
+    return GBO_OK;
+  }
+  void release() {
+    void* all[] = {head, tail, tail_ptr, long_chunk0, chunk_beg, chunk_end, long_row, chunk_row, longbits};
+    for (void* p : all) cudaFree(p);
+  }
+};
+
+int fill_slices(const gbo_graph* g, Slices& sl, cudaStream_t s) {
   const long long rows = (long long)g->nbr * 32;
+  GBO_TRY(sl.make(&sl.tail_ptr, (size_t)rows + 1));
+  GBO_TRY(sl.make(&sl.head, (size_t)rows * kRwsHead));
+  const int grid = (int)std::min<long long>(((long long)g->nbr + 7) / 8, 16LL * num_sms());
   int* len = nullptr;
   long long* tot = nullptr;
   GBO_CUDA_TRY(pool_malloc_async(&len, sizeof(int) * (size_t)rows, s));
-  GBO_CUDA_TRY(pool_malloc_async(&tot, sizeof(long long), s));
-  GBO_CUDA_TRY(cudaMalloc(&g->rws_tail_ptr, sizeof(long long) * (size_t)(rows + 1)));
-  GBO_CUDA_TRY(cudaMalloc(&g->rws_head, sizeof(uint2) * (size_t)rows * kRwsHead));
-  g->device_bytes += 8LL * (rows + 1) + 8LL * rows * kRwsHead;
-  int nsm = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = (int)std::min<long long>(((long long)g->nbr + 7) / 8, 16LL * nsm);
-  k_rws_count<<<grid, 256, 0, s>>>(g->rowptr, g->nbr, g->rowmask, len);
-  GBO_TRY(exclusive_scan_i32_to_i64(len, g->rws_tail_ptr, rows, tot, s));
-  long long nt = 0;
-  GBO_CUDA_TRY(cudaMemcpyAsync(&nt, tot, sizeof(nt), cudaMemcpyDeviceToHost, s));
-  GBO_CUDA_TRY(cudaStreamSynchronize(s));
+  cudaError_t e = pool_malloc_async(&tot, sizeof(long long), s);
+  int st = e == cudaSuccess ? GBO_OK : fail_cuda(e, "row-word slices");
+  if (st == GBO_OK) {
+    k_rws_count<<<grid, 256, 0, s>>>(g->rowptr, g->nbr, g->rowmask, len);
+    st = exclusive_scan_i32_to_i64(len, sl.tail_ptr, rows, tot, s);
+  }
+  if (st == GBO_OK && (e = read_back(&sl.ntail, tot, sizeof(sl.ntail), s)) != cudaSuccess)
+    st = fail_cuda(e, "row-word slice lengths");
   cudaFreeAsync(len, s);
-  cudaFreeAsync(tot, s);
-  GBO_CUDA_TRY(cudaMalloc(&g->rws_tail, sizeof(uint2) * (size_t)(nt > 0 ? nt : 1)));
-  g->rws_ntail = nt;
-  g->device_bytes += 8LL * (nt > 0 ? nt : 1);
-  k_rws_fill<<<grid, 256, 0, s>>>(g->rowptr, g->colind, g->nbr, static_cast<const unsigned*>(g->val),
-                                  g->rws_tail_ptr, g->rws_head, g->rws_tail);
+  if (tot) cudaFreeAsync(tot, s);
+  GBO_TRY(st);
+  GBO_TRY(sl.make(&sl.tail, (size_t)sl.ntail));
+  k_rws_fill<<<grid, 256, 0, s>>>(g->rowptr, g->colind, g->nbr, static_cast<const unsigned*>(g->val), sl.tail_ptr,
+                                  sl.head, sl.tail);
   GBO_CUDA_TRY(cudaGetLastError());
   // long tails cut into chunks (a host pass over the tail offsets, once)
   std::vector<long long> tp((size_t)rows + 1);
-  GBO_CUDA_TRY(cudaMemcpyAsync(tp.data(), g->rws_tail_ptr, sizeof(long long) * tp.size(), cudaMemcpyDeviceToHost, s));
+  GBO_CUDA_TRY(cudaMemcpyAsync(tp.data(), sl.tail_ptr, sizeof(long long) * tp.size(), cudaMemcpyDeviceToHost, s));
   GBO_CUDA_TRY(cudaStreamSynchronize(s));
   std::vector<int> lrow, crow;
   std::vector<unsigned> lbits((size_t)g->nbr, 0u);
   std::vector<long long> lc0, cbeg, cend;
   for (long long i = 0; i < rows; ++i) {
-    const long long len = tp[(size_t)i + 1] - tp[(size_t)i];
-    if (len <= kRwsLongTail) continue;
+    const long long n = tp[(size_t)i + 1] - tp[(size_t)i];
+    if (n <= kRwsLongTail) continue;
     lrow.push_back((int)i);
     lbits[(size_t)(i / 32)] |= 1u << (31 - i % 32);
     lc0.push_back((long long)cbeg.size());
@@ -1322,21 +1349,44 @@ int build_rws(gbo_graph* g, cudaStream_t s) {
     }
   }
   lc0.push_back((long long)cbeg.size());
-  g->rws_nlong = (int)lrow.size();
-  g->rws_nchunk = (long long)cbeg.size();
-  auto up = [&](auto** dst, const auto& src) -> int {
-    const size_t nb = sizeof(src[0]) * (src.empty() ? 1 : src.size());
-    GBO_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(dst), nb));
-    g->device_bytes += (long long)nb;
-    if (!src.empty()) GBO_CUDA_TRY(cudaMemcpy(*dst, src.data(), nb, cudaMemcpyHostToDevice));
-    return GBO_OK;
-  };
-  GBO_TRY(up(&g->rws_long_row, lrow));
-  GBO_TRY(up(&g->rws_long_chunk0, lc0));
-  GBO_TRY(up(&g->rws_chunk_row, crow));
-  GBO_TRY(up(&g->rws_chunk_beg, cbeg));
-  GBO_TRY(up(&g->rws_chunk_end, cend));
-  GBO_TRY(up(&g->rws_longbits, lbits));
+  sl.nlong = (int)lrow.size();
+  sl.nchunk = (long long)cbeg.size();
+  GBO_TRY(sl.upload(&sl.long_row, lrow));
+  GBO_TRY(sl.upload(&sl.long_chunk0, lc0));
+  GBO_TRY(sl.upload(&sl.chunk_row, crow));
+  GBO_TRY(sl.upload(&sl.chunk_beg, cbeg));
+  GBO_TRY(sl.upload(&sl.chunk_end, cend));
+  GBO_TRY(sl.upload(&sl.longbits, lbits));
+  return GBO_OK;
+}
+
+}  // namespace
+
+// Complete and unchanging once the graph has them: built under the graph's
+// lock, all of them or (no memory) none.
+int build_rws(gbo_graph* g, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(g->build_mu);
+  if (g->b != 32 || g->layout != GBO_LAYOUT_ROW || !g->rowmask || g->rws_head || g->nbr <= 0) return GBO_OK;
+  Slices sl;
+  const int st = fill_slices(g, sl, s);
+  if (st != GBO_OK) {
+    cudaStreamSynchronize(s);
+    sl.release();
+    return st;
+  }
+  g->rws_tail = sl.tail;
+  g->rws_ntail = sl.ntail;
+  g->rws_tail_ptr = sl.tail_ptr;
+  g->rws_long_row = sl.long_row;
+  g->rws_long_chunk0 = sl.long_chunk0;
+  g->rws_nlong = sl.nlong;
+  g->rws_chunk_row = sl.chunk_row;
+  g->rws_chunk_beg = sl.chunk_beg;
+  g->rws_chunk_end = sl.chunk_end;
+  g->rws_nchunk = sl.nchunk;
+  g->rws_longbits = sl.longbits;
+  g->rws_head = sl.head;
+  g->device_bytes += sl.bytes;
   return GBO_OK;
 }
 
