@@ -3,8 +3,8 @@
 // The reference loops (algorithm/bfs.cu:508-564, sssp.cu:420-470,
 // pr.cu:449-513, cc.cu:223-287) launch 5-9 kernels per iteration and copy a
 // convergence scalar to the host every iteration.  Here termination is decided
-// on the device: BFS on 32x32 tiles and the PageRank-type loops are one
-// cooperative launch whose blocks meet at grid barriers; the other widths' BFS
+// on the device: BFS on 32x32 tiles is one cooperative launch whose blocks meet
+// at grid barriers, the PageRank-type loops a few of them; the other widths' BFS
 // and the scattered adjoint are a CUDA graph with a conditional WHILE node
 // whose body is one iteration (the last block of its closing kernel, by an
 // atomic ticket, clears the condition); connected components are a fixed
@@ -1149,8 +1149,8 @@ __device__ __forceinline__ double pr_row_update(long long i, double a, const flo
   return norm == 1 ? fabs(d) : d * d;
 }
 
-// The whole PageRank-type loop in one cooperative launch over the row lists
-// (gather.cuh), one block an SM.  Warps take parts in turn, sum their rows and
+// Up to `iters` iterations of a PageRank-type loop in one cooperative launch
+// over the row lists (gather.cuh), one block an SM.  Warps take parts in turn, sum their rows and
 // update those that began in the part; the next part's columns load
 // meanwhile.  Rows that cross parts leave their shares in `head` / `tail` and
 // are finished after a grid barrier, a thread per part they end in; a second
@@ -1168,11 +1168,11 @@ __device__ __forceinline__ double pr_row_update(long long i, double a, const flo
 // (the ranges of low-degree rows finish last).
 __global__ void __launch_bounds__(kGatherTPB, 1)
 k_pr_loop(GatherList gl, float* pr, float* prs, const float* __restrict__ inv, const float* __restrict__ pv, Ctrl* ctrl,
-          double* head, double* tail, unsigned long long limit_ns) {
+          double* head, double* tail, unsigned long long limit_ns, int iters) {
   extern __shared__ __align__(16) unsigned char gather_sh[];
   __shared__ double esh[kGatherWarps];
   volatile Ctrl* vc = ctrl;
-  if (ctrl->done) return;
+  if (ctrl->done || ctrl->bar_err) return;  // the loop ended, or gave up, in an earlier launch
   const unsigned lane = threadIdx.x & 31;
   const int wib = (int)(threadIdx.x >> 5);
   GatherShared& sh = reinterpret_cast<GatherShared*>(gather_sh)[wib];
@@ -1180,7 +1180,8 @@ k_pr_loop(GatherList gl, float* pr, float* prs, const float* __restrict__ inv, c
   const int step = (int)gridDim.x * kGatherWarps;
   const double alpha = ctrl->alpha, add = ctrl->add, adds = ctrl->add_scale, tol = ctrl->tol;
   const double ref = ctrl->ref > 0.0 ? ctrl->ref : 1.0;  // ||w||_1 for the adjoint, else 1
-  const int norm = ctrl->norm, row_scale = ctrl->row_scale, n = gl.nrows, max_iter = ctrl->max_iter;
+  const int norm = ctrl->norm, row_scale = ctrl->row_scale, n = gl.nrows;
+  const int end = min(ctrl->max_iter, ctrl->iter + iters);  // of this launch
   unsigned long long* stamps = ctrl->stamps;
   for (int itn = ctrl->iter;;) {
     const float* x0 = pr + (size_t)(itn & 1) * n;
@@ -1234,16 +1235,16 @@ k_pr_loop(GatherList gl, float* pr, float* prs, const float* __restrict__ inv, c
     if (!grid_barrier(ctrl, limit_ns, &ctrl->err_part[itn % 3][0][0], 8, 16, &err)) return;
     const int it = itn + 1;
     const double m = norm == 2 ? sqrt(err) : err;
-    const bool stop = it >= max_iter || (tol >= 0.0 && m <= tol * ref);
+    const bool met = tol >= 0.0 && m <= tol * ref;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       for (int q = 0; q < 8; ++q) ctrl->err_part[(itn + 2) % 3][q][0] = 0.0;
       vc->iter = it;
       vc->last_err = err;
-      if (stop) vc->done = 1;
+      if (met || it >= vc->max_iter) vc->done = 1;
       if (stamps && it <= kStampCap) stamps[it] = global_ns();
       __threadfence();
     }
-    if (stop) return;
+    if (met || it >= end) return;
     itn = it;
   }
 }
@@ -1970,8 +1971,25 @@ int sssp_impl(gbo_graph* g, int src, uint32_t* d_dist, int* h_iters, cudaStream_
 }
 
 // The PageRank-type loop (pv: the personalization or the adjoint's w, or NULL)
-// after k_pr_init: one cooperative launch, a block an SM.
-int run_pr_loop(gbo_graph* g, AlgoState* a, const float* pv, int max_iter, int cap_iters, int* iters, cudaStream_t s) {
+// after k_pr_init: cooperative launches of a block an SM.
+//
+// A launch holds every SM (1,024 threads of 64 registers a block), so other
+// streams' kernels wait for its end: it takes only as many iterations as fill
+// kSegmentParts parts, about 250 us, or one, and what waits runs between two
+// launches.  A BFS call on 4,000 vertices beside PageRank of R-MAT 20 / R-MAT 22
+// took up to 0.12 / 0.42 ms when the loop was a graph of step kernels, the whole
+// solve (1.8 / 9.0 ms) when it was one launch, and up to 0.5 / 1.0 ms now (two
+// launches of its own, each behind one of these).  A further launch costs 4 us:
+// 20 iterations of R-MAT 20 / 21 / 22 take 2,335 / 4,490 / 9,510 us as one
+// launch and 2,384 / 4,595 / 9,645 so; 30 of R-MAT 18 1,214 and 1,226.
+constexpr long long kSegmentParts = 300000;
+
+// Launches queued before the host looks whether the loop has ended, when it may
+// end early: those past the end return at once.
+constexpr int kSegmentsAhead = 4;
+
+int run_pr_loop(gbo_graph* g, AlgoState* a, const float* pv, int max_iter, int cap_iters, int* iters, cudaStream_t s,
+                float tol) {
   GatherList gl = gather_of(g);
   int per_sm = 0;
   const size_t smem = sizeof(GatherShared) * kGatherWarps;
@@ -1979,7 +1997,7 @@ int run_pr_loop(gbo_graph* g, AlgoState* a, const float* pv, int max_iter, int c
   GBO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_loop, kGatherTPB, smem));
   if (per_sm < 1) return fail(GBO_ERR_UNSUPPORTED, "PageRank loop kernel does not fit an SM");
   // every SM from a few parts a block on (a barrier over few blocks is cheaper)
-  const int grid = std::max(1, std::min((gl.nparts + 3) / 4, num_sms()));
+  int grid = std::max(1, std::min((gl.nparts + 3) / 4, num_sms()));
   const size_t np = (size_t)std::max(gl.nparts, 1);
   if (!a->pr_part) {
     GBO_CUDA_TRY(cudaMalloc(&a->pr_part, sizeof(double) * 2 * np));
@@ -1990,11 +2008,30 @@ int run_pr_loop(gbo_graph* g, AlgoState* a, const float* pv, int max_iter, int c
   Ctrl* ctrl = a->ctrl;
   double *head = a->pr_part, *tail = a->pr_part + np;
   unsigned long long limit_ns = kBarrierLimitNs;
-  void* args[] = {&gl, &pr, &prs, &inv, &pv, &ctrl, &head, &tail, &limit_ns};
-  GBO_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pr_loop, dim3((unsigned)grid), dim3(kGatherTPB), args, smem, s));
-  a->fixed_launches = 2;  // init and the loop
+  int per_launch = (int)std::max(1ll, std::min<long long>(kSegmentParts / (long long)np, max_iter));
+  void* args[] = {&gl, &pr, &prs, &inv, &pv, &ctrl, &head, &tail, &limit_ns, &per_launch};
+  const long long segments = ((long long)max_iter + per_launch - 1) / per_launch;
+  a->fixed_launches = 1;  // init
   a->coop_run = true;
   a->launches_per_iter = 0;
+  for (long long q = 0; q < segments; ++q) {
+    cudaError_t e;
+    // a context or stream that may use fewer SMs refuses the grid: the loop
+    // takes any (the first launch settles it: the barrier counts blocks)
+    while ((e = cudaLaunchCooperativeKernel((const void*)k_pr_loop, dim3((unsigned)grid), dim3(kGatherTPB), args, smem,
+                                            s)) == cudaErrorCooperativeLaunchTooLarge &&
+           q == 0 && grid > 1) {
+      (void)cudaGetLastError();
+      grid = (grid + 1) / 2;
+    }
+    GBO_CUDA_TRY(e);
+    ++a->fixed_launches;
+    if (q + 1 < segments && (q + 1) % kSegmentsAhead == 0 && (tol >= 0.f || cap_iters > 0)) {
+      GBO_CUDA_TRY(cudaMemcpyAsync(a->h_ctrl, a->ctrl, offsetof(Ctrl, err_part), cudaMemcpyDeviceToHost, s));
+      GBO_CUDA_TRY(cudaStreamSynchronize(s));
+      if (a->h_ctrl->done || a->h_ctrl->bar_err) break;
+    }
+  }
   return finish_loop(a, s, max_iter, cap_iters, iters, true);
 }
 
@@ -2013,7 +2050,7 @@ int pr_impl(gbo_graph* g, const float* d_v, float alpha, int max_iter, float tol
                                                   cap_iters);
   GBO_CUDA_TRY(cudaGetLastError());
   int iters = 0;
-  if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_v, max_iter, cap_iters, &iters, s));
+  if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_v, max_iter, cap_iters, &iters, s, tol));
   if (g->nrows > 0)
     GBO_CUDA_TRY(cudaMemcpyAsync(d_p, pr + (size_t)(iters & 1) * g->nrows,
                                  sizeof(float) * (size_t)g->nrows, cudaMemcpyDeviceToDevice, s));
@@ -2042,7 +2079,7 @@ int ppr_backward_impl(gbo_graph* g, const float* d_w, float alpha, float tol, in
                                   0.f, 1.f, 1, 1, a->stamps, cap_iters);
     k_l1_ref<<<gv, kTPB, 0, s>>>(d_w, n, ctrl);
     GBO_CUDA_TRY(cudaGetLastError());
-    if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_w, max_iter, cap_iters, &iters, s));
+    if (max_iter > 0) GBO_TRY(run_pr_loop(g, a, d_w, max_iter, cap_iters, &iters, s, tol));
     if (n > 0) k_scale_copy<<<gv, kTPB, 0, s>>>(pr + (size_t)(iters & 1) * n, d_grad, n, 1.f - alpha);
     GBO_CUDA_TRY(cudaGetLastError());
     if (h_iters) *h_iters = iters;

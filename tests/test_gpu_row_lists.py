@@ -100,3 +100,52 @@ def test_injected_iteration_cap(gbo, gpu):
     finally:
         gbo.debug_inject(gbo.INJECT_REPLAY_CAP, 0)
     assert g.pagerank(0.85, 100)[1] == 100
+
+
+def test_loop_in_several_launches(gbo, gpu):
+    """A loop holds the SMs for a bounded stretch: a large graph's iterations
+    take several launches, with the same result and stopping point."""
+    csr = gbo.gen_rmat(19, 16, seed=5)  # about 70,000 parts
+    n = csr.nrows
+    g = gbo.Graph.from_csr(csr, 32, gbo.FLAG_SYMMETRIC)
+    alpha = float(np.float32(0.85))
+    deg = np.bincount(csr.colind, minlength=n).astype(np.float64)
+    inv = np.divide(1.0, deg, out=np.zeros(n), where=deg > 0)
+    p = np.full(n, 1.0 / n)
+    for _ in range(11):
+        p = alpha * _sum_rows(csr, p * inv) + (1 - alpha) / n
+    got, iters = g.pagerank(alpha, 11)
+    stats = g.last_run()
+    assert iters == 11 and stats["iterations"] == 11 and len(stats["step_ms"]) == 11
+    assert 1 + 2 <= stats["kernel_launches"] <= 1 + 11  # the init kernel and the loop's
+    _check(got.astype(np.float64), p)
+    for tol in (1e-5, 1e-7):
+        early, k = g.pagerank(alpha, 500, tol)
+        assert 1 < k < 500
+        assert np.array_equal(early, g.pagerank(alpha, k)[0])
+
+
+def test_stream_with_a_part_of_the_sms(gbo, gpu):
+    """A stream of a green context of 16 SMs refuses a grid of a block per SM:
+    the loop runs on fewer blocks."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == drv.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    csr = gbo.gen_rmat(16, 16, seed=2)
+    g = gbo.Graph.from_csr(csr, 32, gbo.FLAG_SYMMETRIC)
+    want = g.pagerank(0.85, 7)[0]
+    dev = ok(drv.cuDeviceGet(0))
+    sms = ok(drv.cuDeviceGetDevResource(dev, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    part = ok(drv.cuDevSmResourceSplitByCount(1, sms, 0, 16))[0]
+    ctx = ok(drv.cuGreenCtxCreate(ok(drv.cuDevResourceGenerateDesc([part[0]], 1)), dev,
+                                  drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    s = ok(drv.cuGreenCtxStreamCreate(ctx, drv.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    try:
+        assert np.array_equal(g.pagerank(0.85, 7, stream=int(s))[0], want)
+    finally:
+        drv.cuStreamSynchronize(s)
+        drv.cuStreamDestroy(s)
+        drv.cuGreenCtxDestroy(ctx)
