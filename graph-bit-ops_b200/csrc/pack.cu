@@ -79,12 +79,13 @@ __device__ __forceinline__ void consume(RowCursor& c, const int* __restrict__ co
 }
 
 // Which slabs go to k_pack_wide.  The merge takes a step per tile and, inside
-// it, a turn per entry of the longest run, so a slab is wide when it has more
-// than merge_tiles tiles or a row of more than kMergeRow entries.  The fill
-// pass knows the tiles; the count pass bounds them by the slab's entries
+// it, a turn per entry of the longest run, so a slab may be wide when it has
+// more than merge_tiles tiles or a row of more than kMergeRow entries.  The
+// fill pass knows the tiles; the count pass bounds them by the slab's entries
 // (kMergeEntries, which also keeps short slabs of long rows) and by the block
-// columns between its first and its last one.  k_pack asks and lists the
-// slab's units.
+// columns between its first and its last one, and takes the slab only if the
+// rows' last entries lie in many of these: a mesh's rows lie side by side, seven
+// tiles over any span.  k_pack asks and lists the slab's units.
 // Measured (count and fill, us): the merge alone takes 24,700 on R-MAT 19
 // (16 edges a vertex, b = 32), where block row 0 alone has 16,384 tiles; wide
 // slabs past 48 / 64 / 96 tiles 662 / 660 / 696, and at b = 4 (1,138 / 989 /
@@ -92,12 +93,37 @@ __device__ __forceinline__ void consume(RowCursor& c, const int* __restrict__ co
 // in 92 and would take 185 as wide slabs; a dense 1,100-vertex R-MAT (35
 // tiles, rows of hundreds) merges in 231 and takes 144.  kMergeEntries 128 is
 // for b = 16 meshes (115; 173 at 64 entries) at the cost of 2 % on R-MAT.
+//
+// A wide slab costs its entries and a pass over the bitmap of *all* block
+// columns, so it also needs enough steps for that (words of the bitmap a step,
+// at most: fill_words, count_words) -- or to be a straggler, with more than
+// 1 / kStragglers of the graph's work and kAboveMean times a slab's mean, which
+// the merge would finish last: no more than kStragglers slabs are, so the pass
+// stays linear in the graph.  Where the sides meet (uniform graphs, merge /
+// wide, us): fill b = 4, 2.7 words a tile 75 / 108; b = 8, 2.7 148 / 148; b = 16,
+// 8 265 / 288; b = 32, 10.7 17,525 / 21,143; b = 64, 1.4 15,045 / 15,376; count
+// b = 8, 10.7 words an entry 276 / 201, 42.7 869 / 1,216; b = 16, 42.7 6,141 /
+// 5,020.  Stragglers (R-MAT 19 / 22, b = 8, fill, us): 16,384 and 4 times the
+// mean 741 / 12,857, 32,768 and 2 533 / 17,369, 65,536 and 2 539 / 20,756.
+// Without this rule the fill of uniform graphs of 2^23 vertices, 24 a row, took
+// 2,574 ms at b = 4 and 736 at b = 8 (merge: 4.3, 4.9), the count of a mesh of
+// that size at b = 32 1,299 us (merge: 247).
 constexpr int kMergeEntries = 128;
 constexpr int kMergeRow = 48;
 template <int B>
 __host__ __device__ constexpr int merge_tiles() {
   return B == 4 ? 80 : 48;
 }
+template <int B>
+__host__ __device__ constexpr int fill_words() {
+  return B == 4 ? 1 : B == 8 ? 3 : B == 16 ? 7 : B == 32 ? 10 : 4;
+}
+template <int B>
+__host__ __device__ constexpr int count_words() {
+  return 3 * B;
+}
+constexpr long long kStragglers = 32768;
+constexpr int kAboveMean = 2;
 constexpr int kUnitEntries = 2048;
 
 // Units of a slab with this many entries.
@@ -168,18 +194,31 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
     int longest = c0.end - c0.pos;
     if (M::RPL == 2) longest = max(longest, c1.end - c1.pos);
     longest = -seg_min(-longest, M::W);
-    bool w = slab_ok && entries > kMergeEntries;
+    const long long words = (((long long)ncols + B - 1) / B + 31) / 32;  // of the bitmap
+    const long long stragglers = min(kStragglers, (long long)nbr / kAboveMean);
+    bool w;
     if (BUILD) {
-      w = slab_ok && (bsr_rowptr[slab + 1] - bsr_rowptr[slab] > merge_tiles<B>() || longest > kMergeRow);
-    } else if (__any_sync(0xffffffffu, w)) {
-      int first = c0.head, last = c0.pos < c0.end ? colind[c0.end - 1] : -1;
-      if (M::RPL == 2) {
-        first = min(first, c1.head);
-        last = max(last, c1.pos < c1.end ? colind[c1.end - 1] : -1);
+      const int tiles = slab_ok ? bsr_rowptr[slab + 1] - bsr_rowptr[slab] : 0;
+      const long long steps = max(tiles, longest);
+      w = slab_ok && (tiles > merge_tiles<B>() || longest > kMergeRow) &&
+          (steps * fill_words<B>() >= words || steps * stragglers >= bsr_rowptr[nbr]);
+    } else {
+      const bool straggler = entries * stragglers >= nnz;
+      w = slab_ok && entries > kMergeEntries && (entries * count_words<B>() >= words || straggler);
+      if (__any_sync(0xffffffffu, w)) {
+        int first = c0.head, last = c0.pos < c0.end ? colind[c0.end - 1] : -1;
+        const int before = __shfl_up_sync(0xffffffffu, last / B, 1, M::W);
+        const unsigned moves = __ballot_sync(0xffffffffu, r > 0 && last >= 0 && last / B != before);
+        const int moved = __popc((moves >> (g * M::W)) & (0xffffffffu >> (32 - M::W)));
+        if (M::RPL == 2) {
+          first = min(first, c1.head);
+          last = max(last, c1.pos < c1.end ? colind[c1.end - 1] : -1);
+        }
+        first = seg_min(first, M::W);
+        last = -seg_min(-last, M::W);
+        w = w && (longest > kMergeRow || ((straggler || moved > M::W / 4) &&
+                                          (long long)last / B - (long long)first / B >= merge_tiles<B>()));
       }
-      first = seg_min(first, M::W);
-      last = -seg_min(-last, M::W);
-      w = w && (longest > kMergeRow || (long long)last / B - (long long)first / B >= merge_tiles<B>());
     }
     if (w) {
       if (r == 0) {

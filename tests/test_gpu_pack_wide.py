@@ -115,3 +115,60 @@ def test_errors_past_one_window(gbo, gpu, b, nbc):
         assert e.value.status == status
     ptr, col = _csr(good, ncols)
     _pack(gbo, ptr, col, b, ncols, b, 0)
+
+
+@pytest.mark.parametrize("b", WIDTHS)
+@pytest.mark.parametrize("ncols", [1500, 60_001, 3_000_000])
+def test_slabs_on_both_sides_of_the_rules(gbo, orc, gpu, b, ncols):
+    """One graph of hub slabs, slabs about the rules' lines (steps against the
+    bitmap's words, the share of all work, side-by-side rows as in a mesh) and
+    short ones: every slab is packed alike whoever packs it."""
+    rng = np.random.default_rng(b + ncols)
+    words = (ncols + b - 1) // b // 32 + 1
+    rows = []
+    for slab in range(40):
+        kind = slab % 5
+        steps = [3, words, words // 8, 200, 60][kind] * int(rng.integers(1, 4))
+        for i in range(b):
+            if kind == 4:  # short rows side by side over a wide span
+                at = np.concatenate([slab * b + i + np.arange(-1, 2) + d for d in (0, ncols // 2, ncols - 50 * b)])
+                rows.append(np.unique(at[(at >= 0) & (at < ncols)]))
+            else:
+                k = min(max(2 * steps // b, 1), 20_000 // b + 40, ncols // 2)
+                rows.append(np.unique(rng.integers(0, ncols, k)))
+    ptr, col = _csr(rows, ncols)
+    for layout in (0, 1):
+        ref = orc.pack(ptr, col, len(rows), ncols, b, layout)
+        brp, bci, out = _pack(gbo, ptr, col, len(rows), ncols, b, layout)
+        assert np.array_equal(brp, ref.rowptr) and np.array_equal(bci, ref.colind)
+        assert np.array_equal(out, ref.narrow())
+
+
+@pytest.mark.parametrize("b", [4, 8])
+def test_fill_time_is_linear_in_the_graph(gbo, gpu, b):
+    """A uniform graph four times as large takes about four times as long (16
+    times when every slab walked a bitmap of all block columns)."""
+    torch = pytest.importorskip("torch")
+
+    def fill_ms(n):
+        gen = torch.Generator(device="cuda").manual_seed(n)
+        col = torch.randint(0, n, (n, 24), generator=gen, device="cuda", dtype=torch.int32).sort(1).values.flatten()
+        ptr = torch.arange(0, 24 * n + 1, 24, device="cuda", dtype=torch.int32)
+        rp = torch.empty((n + b - 1) // b + 1, dtype=torch.int32, device="cuda")
+        nb = gbo.C.c_int(0)
+        lib, args = gbo.lib(), (ptr.data_ptr(), col.data_ptr(), n, n, 24 * n, b)
+        torch.cuda.synchronize()
+        gbo.check(lib.gbo_b2sr_nnzb(*args, rp.data_ptr(), gbo.C.byref(nb), None), "nnzb")
+        ci = torch.empty(nb.value, dtype=torch.int32, device="cuda")
+        val = torch.empty(nb.value * b, dtype=torch.uint8, device="cuda")
+        best = float("inf")
+        for _ in range(4):
+            a, z = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            gbo.check(lib.gbo_b2sr_pack(*args, 0, rp.data_ptr(), ci.data_ptr(), val.data_ptr(), None), "pack")
+            z.record()
+            z.synchronize()
+            best = min(best, a.elapsed_time(z))
+        return best
+
+    assert fill_ms(1 << 21) < 12 * fill_ms(1 << 19)
