@@ -214,6 +214,7 @@ extern "C" int gbo_graph_from_csr(const int* rowptr, const int* colind, int nrow
 
   gbo_graph* g = new gbo_graph();
   g->symmetric = (flags & GBO_FLAG_SYMMETRIC) && !lower && nrows == ncols;
+  if (lower) g->tc_lower = 1;
   g->tc_mma = (flags & GBO_FLAG_TC_MMA) != 0;
   if (!perm.empty()) {
     if (cudaMalloc(&g->perm, sizeof(int) * perm.size()) != cudaSuccess ||
@@ -573,6 +574,7 @@ extern "C" int gbo_tune_tile_width(const int* rowptr, const int* colind, int nro
         }
       };
       st = run();
+      if (st == GBO_OK && op == GBO_TUNE_TC) st = run();  // the second count may build what the others read
       float ms = 0.f;
       if (st == GBO_OK) {
         cudaEventRecord(e0, s);

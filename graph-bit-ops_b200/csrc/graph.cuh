@@ -76,6 +76,8 @@ struct gbo_graph {
   int* tc_unit = nullptr;       // the row of every unit
   int* tc_unit0 = nullptr;      // every row's first unit (nrows + 1)
   int tc_nunits = -1;           // -1: not built
+  int tc_lower = -1;            // 1: no entry above the diagonal, 0: some, -1: not known
+  bool tc_counted = false;      // a direct count has run
   int gl_nlong = 0;             // rows of more than kLongRow set bits,
   int gl_nlchunk = 0;           // their chunks (at most kLongChunk set bits each)
   int* gl_long_row = nullptr;   // gl_nlong rows, ascending

@@ -24,16 +24,21 @@
 // entries in place of both: 1,171).  Tiles / lists, us, with the lists built:
 // R-MAT 17 2,679 / 483, ef 24 shuffled b = 16 5,261 / 921, R-MAT 20
 // 75,430 / 7,763, uniform of 100,003 vertices and 24 per vertex b = 8
-// 622 / 103, mesh of 10^6 vertices 121 / 42.  A graph's first call, building
-// included: 3,100 / 1,170, -, 76,000 / 11,600, 1,040 / 400, 530 / 210.
+// 622 / 103, mesh of 10^6 vertices 121 / 42.
 //
-// Building costs 180 us and more however small the graph; the tiles of
-// kListTiles are counted in about 100 (uniform of 10,000 vertices, 65,764
-// tiles: 90, with lists 42, the first call 240; R-MAT of 20,001, 122,369:
-// 347, 54, 410).  Fewer tiles, tensor-core counts and matrices with an entry
-// above the diagonal keep the tile kernels, as does a call under stream capture
-// before the lists are built (nothing can be read back there) or one without
-// memory for them.
+// Building costs 180 us and more however small the graph, and a program may
+// count once.  So a graph's first count goes over lists only where that is no
+// slower than over tiles (from kListFirst tiles on, kListFirstLong where block
+// rows are long: the tile kernel searches them), and from kListTiles on the
+// second count builds them.  First counts, tiles / lists, us (later ones over
+// lists 34 to 100): uniform, 24 a vertex, b = 8, 111,000 tiles 120 / 237, 351,000
+// 257 / 282, 471,000 317 / 288, 591,000 371 / 313; b = 16, 445,000 497 / 284; b =
+// 32, 98,000 273 / 238, 359,000 843 / 305; R-MAT b = 8, 70,000 315 / 319, 122,000
+// 438 / 387, 240,000 695 / 475; mesh b = 8, 99,000 106 / 158, 397,000 213 / 201.
+// Fewer tiles, tensor-core counts and matrices with an entry above the diagonal
+// (looked for before anything is built) keep the tile kernels, as does a call
+// under stream capture before the lists are built (nothing can be read back
+// there) or one without memory for them.
 #include <algorithm>
 
 #include "gather.cuh"
@@ -54,6 +59,10 @@ __device__ __forceinline__ int lower_bound_dev(const int* __restrict__ a, int lo
 }
 
 constexpr long long kListTiles = 1 << 16;
+constexpr long long kListFirst = 1 << 19;
+constexpr long long kListFirstLong = 1 << 17;  // where block rows are long:
+constexpr int kLongMean = 128;                 // tiles of one on average, or
+constexpr int kSkew = 8;                       // the longest against the average
 constexpr int kUnit = 64;       // entries of a list that one warp goes through
 constexpr int kBits = 32768;    // ranks in a warp's bitmap
 constexpr int kPiece = 256;     // entries of a list looked up among at a time
@@ -315,6 +324,25 @@ __global__ void __launch_bounds__(kTPB) k_tc_diagonal(GatherList gl, unsigned lo
     }
   }
   add_count(acc, count);
+}
+
+// Whether some entry lies above the diagonal: a thread per block row looks at
+// its last tile (block columns ascend).
+template <int B>
+__global__ void k_above(GView v, unsigned* __restrict__ above) {
+  using WT = typename Word<B>::T;
+  const int R = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  bool up = false;
+  if (R < v.nbr && v.rowptr[R + 1] > v.rowptr[R]) {
+    const int t = v.rowptr[R + 1] - 1, C = v.colind[t];
+    up = C > R;
+    if (C == R) {
+      const WT* __restrict__ w = reinterpret_cast<const WT*>(v.val) + (size_t)t * B;
+#pragma unroll 8
+      for (int r = 0; r < B; ++r) up = up || (w[r] & (WT)(((WT)1 << (B - 1 - r)) - 1));
+    }
+  }
+  if (__any_sync(0xffffffffu, up) && (threadIdx.x & 31) == 0) *above = 1u;
 }
 
 // Block row of every tile, from the work items.
@@ -671,22 +699,49 @@ bool capturing(cudaStream_t s) {
   return cap != cudaStreamCaptureStatusNone;
 }
 
+// Fills in g->tc_lower.
+int find_lower(gbo_graph* g, cudaStream_t s) {
+  if (g->tc_lower >= 0) return GBO_OK;
+  unsigned *d = nullptr, h = 0;
+  GBO_CUDA_TRY(pool_malloc_async(&d, sizeof(unsigned), s));
+  const GView v = view_of(g);
+  const unsigned grid = blocks_for(g->nbr, 256);
+  cudaError_t e = cudaMemsetAsync(d, 0, sizeof(unsigned), s);
+  switch (g->b) {
+    case 4: k_above<4><<<grid, 256, 0, s>>>(v, d); break;
+    case 8: k_above<8><<<grid, 256, 0, s>>>(v, d); break;
+    case 16: k_above<16><<<grid, 256, 0, s>>>(v, d); break;
+    case 32: k_above<32><<<grid, 256, 0, s>>>(v, d); break;
+    default: k_above<64><<<grid, 256, 0, s>>>(v, d); break;
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = read_back(&h, d, sizeof(h), s);
+  cudaFreeAsync(d, s);
+  if (e != cudaSuccess) return fail_cuda(e, "triangle of a matrix");
+  g->tc_lower = h ? 0 : 1;
+  return GBO_OK;
+}
+
 // Whether the count goes over lists, which are built if need be.
 bool lists_ready(gbo_graph* g, cudaStream_t s, bool may_build, int* st) {
   if (g->tc_mma || g->nblk < kListTiles) return false;
-  if (g->gl_nparts < 0 && !may_build) return false;
-  *st = build_gather(g, s);
-  if (*st == GBO_OK && !g->gl_lower) return false;
-  if (*st == GBO_OK && !counted_by_lane(g)) {
-    if (g->tc_nunits < 0 && !may_build) return false;
-    *st = build_lists(g, s);
+  const bool first = !g->tc_counted;
+  if (may_build) {
+    g->tc_counted = true;
+    const bool lng = g->nblk > (long long)kLongMean * g->nbr || (long long)g->longest * g->nbr > kSkew * g->nblk;
+    if (first && g->nblk < (lng ? kListFirstLong : kListFirst)) return false;
+    *st = find_lower(g, s);
+    if (*st == GBO_OK && g->tc_lower) *st = build_gather(g, s);
+    if (*st == GBO_OK && g->tc_lower && !counted_by_lane(g)) *st = build_lists(g, s);
+    if (*st == GBO_ERR_NOMEM) {
+      clear_error();
+      *st = GBO_OK;
+      return false;
+    }
+    return *st == GBO_OK && g->tc_lower == 1;
   }
-  if (*st == GBO_ERR_NOMEM) {
-    clear_error();
-    *st = GBO_OK;
-    return false;
-  }
-  return *st == GBO_OK;
+  // under capture: what direct counts have built
+  return g->tc_lower == 1 && g->gl_nparts >= 0 && (counted_by_lane(g) || g->tc_nunits >= 0);
 }
 
 // The tiles' block rows: made by the first direct count, complete when it goes

@@ -363,11 +363,11 @@ GBO_API int gbo_cc(const gbo_graph* g, int32_t* d_label, int* h_iters,
  * result (bsrbmm/bsrbmm.cu:1214-1265, 1416; bsrbmm/tc.cu:767-951). */
 GBO_API int gbo_tc(const gbo_graph* lower, uint64_t* h_count, gbo_stream_t stream);
 /* Same, result left in device memory (*d_count is overwritten).  Returns once
- * queued, except that a graph's first count derives what the counts read (the
- * tiles' block rows; neighbour lists from 65,536 tiles on) and waits for the
- * stream.  Under stream capture it always just queues: a graph not counted
- * directly before is counted over its tiles, whose block rows the captured
- * graph then derives on each launch. */
+ * queued, except that a graph's first and second count may derive what the
+ * counts read (the tiles' block rows; from 65,536 tiles on neighbour lists) and
+ * then wait for the stream.  Under stream capture it always just queues: a graph
+ * not counted directly before is counted over its tiles, whose block rows the
+ * captured graph then derives on each launch. */
 GBO_API int gbo_tc_device(const gbo_graph* lower, unsigned long long* d_count,
                   gbo_stream_t stream);
 

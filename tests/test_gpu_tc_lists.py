@@ -91,3 +91,40 @@ def test_wrapped_graph_with_wrong_degrees(gbo, orc, gpu, b):
     assert g.info().nblocks >= TILES
     for _ in range(2):
         assert g.tc() == want
+
+
+@pytest.mark.parametrize("kind,n,b,first", [("mesh", 700_569, 8, False), ("sparse", 90_001, 8, False),
+                                            ("dense", 40_001, 64, True), ("sparse", 600_001, 8, True)])
+def test_first_count_builds_where_it_pays(gbo, orc, gpu, kind, n, b, first):
+    """A graph's first count goes over the tiles where building the lists would
+    cost more; its second one builds them."""
+    rowptr, colind = _lower(gbo, kind, n, False)
+    want = orc.tc_b2sr(orc.pack(rowptr, colind, n, n, b))
+    g = gbo.Graph.from_csr(gbo.Csr(rowptr, colind, n, n), b)
+    before = g.info()
+    assert before.nblocks >= TILES
+    assert g.tc() == want
+    lists = 4 * len(colind) + 8 * n
+    assert (g.info().device_bytes >= before.device_bytes + lists) == first
+    assert g.tc() == want
+    assert g.info().device_bytes >= before.device_bytes + lists
+
+
+@pytest.mark.parametrize("b", [4, 8, 16, 32, 64])
+@pytest.mark.parametrize("where", ["diagonal_tile", "above_it"])
+def test_one_entry_above_builds_nothing(gbo, orc, gpu, b, where):
+    n = 40_001
+    rowptr, colind = _lower(gbo, "dense", n, True)
+    row = np.repeat(np.arange(n), np.diff(rowptr))
+    at = b * (n // b // 2)
+    extra = at * n + (at + b - 1 if where == "diagonal_tile" else at + b)
+    key = np.unique(np.concatenate([row * np.int64(n) + colind, [extra]]))
+    rowptr = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(key // n, minlength=n), out=rowptr[1:])
+    colind = (key % n).astype(np.int32)
+    want = orc.tc_b2sr(orc.pack(rowptr, colind, n, n, b))
+    g = gbo.Graph.from_csr(gbo.Csr(rowptr, colind, n, n), b)
+    before = g.info()
+    for _ in range(3):
+        assert g.tc() == want
+    assert g.info().device_bytes == before.device_bytes + 4 * before.nblocks  # the tiles' block rows
