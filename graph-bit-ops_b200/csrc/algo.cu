@@ -1374,8 +1374,9 @@ __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ 
 // Afforest (Sutton, Ben-Nun, Barak, "Optimizing Parallel Graph Connectivity
 // Computation via Subgraph Sampling", IPDPS 2018) over the row lists: a
 // forest in the caller's label array whose links always go from a higher to a
-// lower vertex, so a component's root is its smallest vertex.  Two edges per
-// vertex link most of a graph's largest component; a sample of the labels
+// lower vertex, so a component's root is its smallest vertex.  Three edges per
+// vertex (its first, last and second neighbour) link most of a graph's largest
+// component; a sample of the labels
 // names it, and only the vertices outside it go through all their edges (an
 // edge between the two sides is seen from the outside one: P is symmetric).
 //
@@ -1431,13 +1432,24 @@ struct CcState {
   int hooked;
 };
 
+// Passes over the edges so far and the time; one thread.
+__device__ __forceinline__ void cc_pass_done(Ctrl* ctrl, int passes) {
+  ctrl->iter = passes;
+  ctrl->stamps[passes] = global_ns();
+}
+
 // Every vertex under its first neighbour where that is lower (a forest: links
 // go down), so the first edge costs no atomic.
-__global__ void k_cc_init(GatherList gl, int* __restrict__ comp, CcState* __restrict__ st) {
+__global__ void k_cc_init(GatherList gl, int* __restrict__ comp, CcState* __restrict__ st, Ctrl* __restrict__ ctrl,
+                          unsigned long long* stamps) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
     st->list[0] = st->list[1] = 0ull;
     st->hooked = 0;
+    ctrl->done = 0;
+    ctrl->bar_err = 0u;
+    ctrl->stamps = stamps;
+    cc_pass_done(ctrl, 0);
   }
   for (long long v = i; v < gl.nrows; v += (long long)gridDim.x * blockDim.x) {
     const long long b = gl.ptr[v], e = gl.ptr[v + 1];
@@ -1470,7 +1482,8 @@ __global__ void k_cc_hook(GatherList gl, int* comp, int pick) {
 // thread doubles its own vertex's pointer, reading from L2 what the others
 // have doubled so far, so a path of d vertices takes about log d turns (read
 // through L1 it is walked: a mesh's paths of 1,000 took 392 us, now 34).
-__global__ void k_cc_compress(int* comp, int n, const CcState* __restrict__ if_hooked) {
+__global__ void k_cc_compress(int* comp, int n, const CcState* __restrict__ if_hooked, Ctrl* __restrict__ ctrl) {
+  if (if_hooked && blockIdx.x == 0 && threadIdx.x == 0) cc_pass_done(ctrl, 2);
   if (if_hooked && !if_hooked->hooked) return;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
     int p = __ldca(comp + v);
@@ -1483,7 +1496,14 @@ __global__ void k_cc_compress(int* comp, int n, const CcState* __restrict__ if_h
 }
 
 // The labels: every vertex's root, each vertex written by its own thread only.
-__global__ void k_cc_labels(int* comp, int n, const CcState* __restrict__ st) {
+// `passes` lies in page-locked host memory (a copy behind the kernel took 8 us).
+__global__ void k_cc_labels(int* comp, int n, const CcState* __restrict__ st, Ctrl* __restrict__ ctrl,
+                            int* __restrict__ passes) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (st->hooked) cc_pass_done(ctrl, 3);
+    ctrl->done = 1;
+    *passes = st->hooked ? 3 : 2;
+  }
   if (!st->hooked) return;  // the trees are flat
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
     int r = __ldca(comp + v);
@@ -1495,7 +1515,7 @@ __global__ void k_cc_labels(int* comp, int n, const CcState* __restrict__ st) {
 // The most frequent label among the ends of kCcSamples set bits (a wrong guess
 // costs time only).
 __global__ void __launch_bounds__(kCcSamples) k_cc_sample(GatherList gl, const int* __restrict__ comp,
-                                                          CcState* __restrict__ st) {
+                                                          CcState* __restrict__ st, Ctrl* __restrict__ ctrl) {
   __shared__ int lab[kCcSamples];
   __shared__ unsigned best;
   const int t = (int)threadIdx.x;
@@ -1509,7 +1529,10 @@ __global__ void __launch_bounds__(kCcSamples) k_cc_sample(GatherList gl, const i
   for (int q = 0; q < kCcSamples; ++q) c += lab[q] == mine;
   if (mine >= 0) atomicMax(&best, (c << 16) | (unsigned)t);  // count, then any of its holders
   __syncthreads();
-  if (t == 0) st->largest = best ? lab[best & 0xffffu] : -1;
+  if (t == 0) {
+    st->largest = best ? lab[best & 0xffffu] : -1;
+    cc_pass_done(ctrl, 1);
+  }
 }
 
 // Vertices outside the sampled component: all their edges.  Short rows a lane
@@ -2128,32 +2151,35 @@ int cc_impl(gbo_graph* g, int32_t* d_label, int* h_iters, cudaStream_t s) {
   }
   auto* st = static_cast<CcState*>(a->cc);
   auto* list = reinterpret_cast<long long*>(st + 1);
+  Ctrl* ctrl = a->ctrl;
   a->step_ms.clear();
   a->stats_pending = false;
   a->coop_run = false;
   a->replays = 0;
   a->launches = 0;
+  a->launches_per_iter = 0;
   a->h_ctrl->iter = 0;
   if (n > 0) {
     const unsigned gv = grid_vertex(n);
     const bool longs = gl.nnz > kCcChunk;
     const unsigned gc = longs ? grid_persistent(k_cc_long<true>, gl.nnz / kCcChunk + 1) : 0u;
-    k_cc_init<<<gv, kTPB, 0, s>>>(gl, d_label, st);
+    k_cc_init<<<gv, kTPB, 0, s>>>(gl, d_label, st, ctrl, a->stamps);
     for (const int pick : {-1, 1}) {
-      k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr);
+      k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr, ctrl);
       k_cc_hook<<<gv, kTPB, 0, s>>>(gl, d_label, pick);
     }
-    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr);
-    k_cc_sample<<<1, kCcSamples, 0, s>>>(gl, d_label, st);
+    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, nullptr, ctrl);
+    k_cc_sample<<<1, kCcSamples, 0, s>>>(gl, d_label, st, ctrl);
     k_cc_rest<false><<<gv, kTPB, 0, s>>>(gl, d_label, st, list);
     if (longs) k_cc_long<false><<<gc, kTPB, 0, s>>>(gl, d_label, st, list);
-    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, st);
+    k_cc_compress<<<gv, kTPB, 0, s>>>(d_label, n, st, ctrl);
     k_cc_rest<true><<<gv, kTPB, 0, s>>>(gl, d_label, st, list);
     if (longs) k_cc_long<true><<<gc, kTPB, 0, s>>>(gl, d_label, st, list);
-    k_cc_labels<<<gv, kTPB, 0, s>>>(d_label, n, st);
+    k_cc_labels<<<gv, kTPB, 0, s>>>(d_label, n, st, ctrl, &a->h_ctrl->iter);
     GBO_CUDA_TRY(cudaGetLastError());
-    a->launches = 11 + (longs ? 2 : 0);
-    a->h_ctrl->iter = 2;  // the sampled edges, the rest
+    a->fixed_launches = 11 + (longs ? 2 : 0);
+    a->launches = a->fixed_launches;
+    a->stats_pending = true;
   }
   if (h_iters) {
     GBO_CUDA_TRY(cudaStreamSynchronize(s));

@@ -354,7 +354,9 @@ GBO_API int gbo_pagerank(const gbo_graph* g, float alpha, int max_iter, float to
 /* Connected components (P symmetric): label[i] = smallest vertex id in the
  * component of i -- the fixed point of the reference's FastSV loop
  * (algorithm/cc.cu:223-287).  h_iters (nullable) receives the number of
- * passes over the edges; the call then waits for the stream. */
+ * passes over the edges -- a few of every vertex, those of the vertices outside
+ * the largest component found so, and these again where the second pass met two
+ * trees: 2 or 3 -- and the call then waits for the stream. */
 GBO_API int gbo_cc(const gbo_graph* g, int32_t* d_label, int* h_iters,
            gbo_stream_t stream);
 /* Triangles of an undirected simple graph given its lower triangle L
@@ -635,7 +637,8 @@ GBO_API int gbo_gen_er_batch(int count, int nmin, int nmax, double avg_degree,
  *       GBO_ERR_NOMEM and leaves its output untouched;
  *   GBO_INJECT_REPLAY_CAP  (n >= 1) the iteration loops (BFS, SSSP,
  *       PageRank, PPR) run at most 8 n iterations and return
- *       GBO_ERR_TIMEOUT when the device has not finished by then;
+ *       GBO_ERR_TIMEOUT when the device has not finished by then (connected
+ *       components take three passes at most, within any cap);
  *   GBO_INJECT_SERVER_HOLD (n = 1) server workers admit no new query:
  *       submissions stay pending (queries already in flight finish);
  *   GBO_INJECT_BARRIER_SKIP (n >= 1) the next cooperative BFS launch (one

@@ -74,3 +74,19 @@ def test_labels_without_waiting(gbo, orc, gpu):
     for _ in range(3):
         gbo.check(gbo.lib().gbo_cc(g.h, out.ptr, None, s.ptr), "cc")
         assert np.array_equal(out.to_numpy(np.int32, csr.nrows, s.ptr), want)
+
+
+@pytest.mark.parametrize("kind,passes", [(0, 2), (5, 3), ("sparse", 3)])
+def test_passes_and_their_times(gbo, gpu, kind, passes):
+    """h_iters and the run's statistics tell the passes that ran: a star about
+    vertex 0 is one tree after the first edges; about vertex 5 it is not (its
+    second neighbour is taken there, 2 to 4 are left), nor is a sparse random
+    graph."""
+    n = 100_003
+    rng = np.random.default_rng(3)
+    src, dst = rng.integers(0, n, (2, 3 * n // 2)) if kind == "sparse" else (np.full(n, kind), np.arange(n))
+    g = gbo.Graph.from_csr(gbo.csr_from_edges(src, dst, n, True, True), 32)
+    assert g.cc()[1] == passes
+    run = g.last_run()
+    assert run["iterations"] == passes and len(run["step_ms"]) == passes
+    assert min(run["step_ms"]) > 0 and run["kernel_launches"] >= 11
