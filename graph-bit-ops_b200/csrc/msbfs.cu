@@ -177,7 +177,8 @@ int msbfs_impl(gbo_graph* g, MsState& m, const int* h_srcs, int k, int32_t* d_le
     GBO_TRY(live_rows(g, s, &lv));
     m.live = static_cast<const uint32_t*>(lv);
   }
-  GBO_TRY(build_rws(g, s));
+  // the slices carry the levels of k <= 64 and, on symmetric graphs, pushes
+  if (kw <= 2 || g->symmetric) GBO_TRY(build_rws(g, s));
   if (!m.active) {
     GBO_CUDA_TRY(cudaMalloc(&m.active, sizeof(uint32_t) * 64));
     m.slot_any = m.active + 32;
@@ -196,12 +197,8 @@ int msbfs_impl(gbo_graph* g, MsState& m, const int* h_srcs, int k, int32_t* d_le
     m.kw = 0;
     GBO_CUDA_TRY(cudaMalloc(&m.F, sizeof(uint32_t) * 2 * (size_t)n * kw + 16));
     GBO_CUDA_TRY(cudaMalloc(&m.V, sizeof(uint32_t) * (size_t)n * kw + 16));
-    GBO_TRY(ms::split_state(g, kw, &m.split_acc, &m.slot_split, s));
-    if (kw <= 2 || (g->symmetric && g->rws_head)) {  // push levels' accumulator, zero between levels
-      const size_t pw = (size_t)(g->nbr > 0 ? g->nbr : 1) * 32 * (size_t)kw;
-      GBO_CUDA_TRY(cudaMalloc(&m.push_acc, sizeof(uint32_t) * pw));
-      GBO_CUDA_TRY(cudaMemsetAsync(m.push_acc, 0, sizeof(uint32_t) * pw, s));
-    }
+    // only the step over tiles leaves split rows to the finish kernel
+    if (kw <= 2 && !g->rws_head) GBO_TRY(ms::split_state(g, kw, &m.split_acc, &m.slot_split, s));
     const size_t lw = kw > 2 ? (size_t)std::max(g->gl_nlong, 1) * kw : (size_t)std::max(g->rws_nlong, 1) * 2;
     if (lw > m.long_words) {
       cudaFree(m.long_acc);
@@ -212,6 +209,13 @@ int msbfs_impl(gbo_graph* g, MsState& m, const int* h_srcs, int k, int32_t* d_le
     }
     GBO_CUDA_TRY(cudaMemsetAsync(m.long_acc, 0, sizeof(uint32_t) * lw, s));
     m.kw = kw;
+  }
+  // push levels' accumulator, zero between levels (the graph may have become
+  // symmetric since the last call: gbo_graph_set_bfs_direction)
+  if (!m.push_acc && (kw <= 2 || (g->symmetric && g->rws_head))) {
+    const size_t pw = (size_t)(g->nbr > 0 ? g->nbr : 1) * 32 * (size_t)kw;
+    GBO_CUDA_TRY(cudaMalloc(&m.push_acc, sizeof(uint32_t) * pw));
+    GBO_CUDA_TRY(cudaMemsetAsync(m.push_acc, 0, sizeof(uint32_t) * pw, s));
   }
   if (k > m.ksrc) {
     cudaFree(m.srcs);

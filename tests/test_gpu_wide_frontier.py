@@ -36,3 +36,26 @@ def test_levels(gbo, orc, gpu, graphs, k):
         want = np.stack([orc.bfs_csr(csr.rowptr, csr.colind, n, int(s))[0] for s in srcs], 1)
         assert np.array_equal(lv, want)
         assert depth == int(want.max()) + 1
+
+
+def test_directed_graph_builds_no_slices(gbo, gpu, graphs):
+    csr = graphs[0]
+    g = gbo.Graph.from_csr(csr, 32)
+    before = g.info().device_bytes
+    g.msbfs(np.arange(100, dtype=np.int32))
+    slices = 8 * 8 * csr.nrows  # their heads alone
+    assert g.info().device_bytes < before + slices
+
+
+@pytest.mark.parametrize("k", [60, 100, 1000])
+def test_symmetry_asserted_between_calls(gbo, orc, gpu, graphs, k):
+    """A graph that pulled at first pushes once it is said to be symmetric, and
+    pulls again afterwards."""
+    csr = graphs[1]
+    n = csr.nrows
+    srcs = np.arange(5, 5 + k, dtype=np.int32)
+    want = np.stack([orc.bfs_csr(csr.rowptr, csr.colind, n, int(s))[0] for s in srcs], 1)
+    g = gbo.Graph.from_csr(csr, 32)
+    for symmetric, threshold in ((0, -1), (1, -1), (1, 100_000), (0, -1), (1, 50)):
+        g.set_bfs_direction(symmetric, threshold)
+        assert np.array_equal(g.msbfs(srcs)[0], want)
