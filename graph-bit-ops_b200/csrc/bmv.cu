@@ -133,18 +133,27 @@ __device__ __forceinline__ void tile_counts(const void* __restrict__ val, long l
   }
 }
 
-template <int B, bool OUTF, bool WHOLE>
+// What a warp counts: a work item; a whole row, taken by its first item; a block row.
+enum CountBy { kByItem, kByFirstItem, kByRow };
+
+template <int B, bool OUTF, CountBy BY>
 __global__ void __launch_bounds__(kTPB) k_count_narrow(GView v, const typename Word<B>::T* __restrict__ x,
                                                        void* __restrict__ yv, int accumulate,
                                                        int* __restrict__ scratch) {
   const unsigned lane = threadIdx.x & 31;
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (item >= v.nitems) return;
-  gbo_item it = v.items[item];
-  if (WHOLE && it.slot >= 0) {  // the first item takes the row
-    const int r0 = v.rowptr[it.row];
-    if (it.t0 != r0) return;
-    it = gbo_item{it.row, r0, v.rowptr[it.row + 1], -1};
+  gbo_item it;
+  if (BY == kByRow) {
+    if (item >= v.nbr) return;
+    it = gbo_item{(int)item, v.rowptr[item], v.rowptr[item + 1], -1};
+  } else {
+    if (item >= v.nitems) return;
+    it = v.items[item];
+    if (BY == kByFirstItem && it.slot >= 0) {
+      const int r0 = v.rowptr[it.row];
+      if (it.t0 != r0) return;
+      it = gbo_item{it.row, r0, v.rowptr[it.row + 1], -1};
+    }
   }
   unsigned c[B];
 #pragma unroll
@@ -427,14 +436,22 @@ unsigned grid_items(const GView& v) {
 
 // ------------------------------------------------------------- launchers
 template <int B>
-int count_impl(const GView& v, int longest, const void* x, void* y, int out_type, int accumulate,
+int count_impl(const GView& v, long long nblk, int longest, const void* x, void* y, int out_type, int accumulate,
                int* scratch, cudaStream_t s) {
   using WT = typename Word<B>::T;
   // A warp counts chunk_for(B) narrow tiles in less than a second launch takes:
   // where no block row has more, rows are not split (R-MAT of 5,001 rows,
   // b = 16: 8.2 us with the launch, 6.2 without; of 20,001 rows, b = 8, some
   // of 2,501 tiles: 10.3 split, 14.3 with the rows up to 1,024 tiles whole).
-  const bool whole = longest <= chunk_for(B);
+  // A row's first item takes it then; but the other items' warps hold their
+  // block's registers while it runs, so rows of about one length get a warp each
+  // (uniform of 28,590 rows, 24 a row, b = 16: 12.9 us by items, 8.7 by rows).  A
+  // long row among short ones is better off in a block of such idle warps (R-MAT
+  // of 9,001 rows, b = 4: 8.7 by items, 10.8 by rows).  Where no row is split the
+  // forms do the same and their code decides (uniform of 400,003 rows, 24 a row,
+  // by item / by first item: b = 4 32.7 / 31.0, b = 8 34.9 / 33.1, b = 16 62.6 / 67.8).
+  const bool whole = longest <= chunk_for(B) && (B < 16 || v.nsplit > 0);
+  const bool by_row = whole && v.nsplit > 0 && (long long)longest * v.nbr <= 4 * nblk;
   bool narrow = false;
   if (v.nitems > 0) {
     // whole-tile loads need the tile array aligned to a tile (4, 8 or 16
@@ -443,15 +460,18 @@ int count_impl(const GView& v, int longest, const void* x, void* y, int out_type
       constexpr uintptr_t kAlign = B == 4 ? 4 : B == 8 ? 8 : 16;
       narrow = (reinterpret_cast<uintptr_t>(v.val) % kAlign) == 0;
       if (narrow) {
-        const unsigned grid = blocks_for_warps(v.nitems, kTPB / 32);
-        auto run = [&](auto f32, auto rows) {
-          k_count_narrow<B, decltype(f32)::value, decltype(rows)::value>
+        const unsigned grid = blocks_for_warps(by_row ? v.nbr : v.nitems, kTPB / 32);
+        auto run = [&](auto f32, auto by) {
+          k_count_narrow<B, decltype(f32)::value, decltype(by)::value>
               <<<grid, kTPB, 0, s>>>(v, (const WT*)x, y, accumulate, scratch);
         };
-        const std::true_type yes;
-        const std::false_type no;
-        if (out_type == GBO_OUT_F32) whole ? run(yes, yes) : run(yes, no);
-        else whole ? run(no, yes) : run(no, no);
+        auto pick = [&](auto f32) {
+          if (by_row) run(f32, std::integral_constant<CountBy, kByRow>{});
+          else if (whole) run(f32, std::integral_constant<CountBy, kByFirstItem>{});
+          else run(f32, std::integral_constant<CountBy, kByItem>{});
+        };
+        if (out_type == GBO_OUT_F32) pick(std::true_type{});
+        else pick(std::false_type{});
       }
     }
     if (!narrow) {
@@ -590,7 +610,7 @@ int bmv_count(const gbo_graph* g, const void* x, void* y, int out_type, int accu
               void* scratch, cudaStream_t s) {
   GView v = view_of(g);
   int st = GBO_OK;
-  GBO_DISPATCH_B(g->b, st = count_impl<B>(v, g->longest, x, y, out_type, accumulate, (int*)scratch, s));
+  GBO_DISPATCH_B(g->b, st = count_impl<B>(v, g->nblk, g->longest, x, y, out_type, accumulate, (int*)scratch, s));
   return st;
 }
 

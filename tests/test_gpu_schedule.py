@@ -64,3 +64,29 @@ def test_products(gbo, orc, gpu, b, tiles):
     sums = np.bincount(row, weights=xf[csr.colind], minlength=n)
     g.bmv_float(dxf, dy, 1.0, None, 0.0)
     assert np.array_equal(dy.to_numpy(np.float32, n), sums.astype(np.float32))
+
+
+@pytest.mark.parametrize("b", [4, 8, 16])
+def test_counts_of_rows_of_one_length(gbo, orc, gpu, b):
+    """Every block row is cut, none is longer than the others: a warp counts one."""
+    n = 200 * b + b // 2 + 1
+    rng = np.random.default_rng(b)
+    row = np.repeat(np.arange(n), 160)
+    key = np.unique(row * np.int64(n) + rng.integers(0, n, len(row)))
+    key = key[(key // n) // b != 7]  # one block row is empty
+    rowptr = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(key // n, minlength=n), out=rowptr[1:])
+    csr = gbo.Csr(rowptr, (key % n).astype(np.int32), n, n)
+    g, ref = gbo.Graph.from_csr(csr, b), orc.pack(csr.rowptr, csr.colind, n, n, b)
+    assert g.info().nsplit_rows == g.info().nblockrows - 1
+    xw = orc.pack_vector((rng.random(n) < 0.5).astype(np.int32), b)
+    dx = gbo.DeviceBuffer.from_numpy(xw.astype(gbo.WORD_DTYPE[b]))
+    want = orc.bmv_count(ref, xw)
+    dy = gbo.DeviceBuffer.from_numpy(np.full(n, -7, np.int32))
+    g.bmv_count(dx, dy)
+    assert np.array_equal(dy.to_numpy(np.int32, n), want)
+    g.bmv_count(dx, dy, accumulate=True)
+    assert np.array_equal(dy.to_numpy(np.int32, n), 2 * want)
+    df = gbo.DeviceBuffer.from_numpy(np.full(n, 0.5, np.float32))
+    g.bmv_count(dx, df, gbo.OUT_F32, accumulate=True)
+    assert np.array_equal(df.to_numpy(np.float32, n), want + np.float32(0.5))
