@@ -513,14 +513,19 @@ __global__ void k_terms(const float* __restrict__ x, const float* __restrict__ s
     z[j] = x[j] * scale[j];
 }
 
-// Where columns are met several times each, the terms are laid out first and
-// a set bit takes one gather instead of two (R-MAT 20, b = 32: 503 -> 479 us;
-// R-MAT 18, b = 64: 601 -> 558); under 2^20 tiles the launch costs as much
-// (R-MAT of 20,001 rows, b = 8: 33 -> 37).  The buffer comes from the pool, which a stream under
-// capture does not take.  (Degrees are not read ahead: a row pointer need
-// only reach as far as the set columns.)
-float* float_terms(const GView& v, long long nblk, const float* x, const float* scale, cudaStream_t s) {
-  if (!scale || v.ncols <= 0 || nblk < std::max(4ll * v.ncols, 1ll << 20)) return nullptr;
+// Where the gathers of x and scale are what a product waits for -- wide tiles
+// (b = 64) and long block rows among short ones -- the terms are laid out first
+// and a set bit takes one gather instead of two: R-MAT 20, b = 32 492 -> 476 us,
+// b = 64 2,614 -> 2,520; R-MAT of 150,001 rows, b = 16 195 -> 184.  Else the
+// gathers hide behind the words, and the launch is lost: uniform of 60,001 rows,
+// 24 a row, b = 4 42.0 -> 45.9, b = 32 29.2 -> 33.4; of 1,048,576 rows, b = 32
+// 323 -> 324.  The same holds for few tiles.  The buffer comes from the pool,
+// which a stream under capture does not take.  (Degrees are not read ahead: a
+// row pointer need only reach as far as the set columns.)
+float* float_terms(const gbo_graph* g, const GView& v, const float* x, const float* scale, cudaStream_t s) {
+  const bool skewed = (long long)g->longest * g->nbr > 12 * g->nblk;
+  const long long least = g->b >= 16 && skewed ? 1ll << 20 : g->b == 64 ? 1ll << 21 : 1ll << 62;
+  if (!scale || v.ncols <= 0 || g->nblk < least) return nullptr;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   float* z = nullptr;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
@@ -642,7 +647,7 @@ int bmv_float(const gbo_graph* g, const float* x, float* y, float alpha, const f
               float add, void* scratch, cudaStream_t s, const int* degptr) {
   GView v = view_of(g);
   SrParams p{alpha, add, scale, degptr};
-  float* z = degptr ? nullptr : float_terms(v, g->nblk, x, scale, s);
+  float* z = degptr ? nullptr : float_terms(g, v, x, scale, s);
   if (z) {
     x = z;
     p.scale = nullptr;

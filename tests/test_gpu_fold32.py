@@ -62,3 +62,23 @@ def test_terms_beforehand(gbo, orc, gpu, b):
     csr = _csr(gbo, src, dst, n)
     assert gbo.Graph.from_csr(csr, b).info().nblocks >= max(1 << 20, 4 * n)
     _check(gbo, orc, csr, b, rng)
+
+
+@pytest.mark.parametrize("b", [8, 16, 32, 64])
+def test_terms_beforehand_on_a_skewed_graph(gbo, gpu, b):
+    """A million tiles and a hub row far past the others (b = 8: not laid out)."""
+    rng = np.random.default_rng(b)
+    n = 300_007
+    src = np.concatenate([rng.integers(0, n, 1_150_000), np.full(n, 77)])
+    dst = np.concatenate([rng.integers(0, n, 1_150_000), np.arange(n)])
+    csr = _csr(gbo, src, dst, n)
+    g = gbo.Graph.from_csr(csr, b)
+    info = g.info()
+    assert info.nblocks >= 1 << 20 and info.nblockcols * info.nblockrows > 12 * info.nblocks
+    x, scale = rng.integers(0, 8, n).astype(np.float32), rng.integers(1, 4, n).astype(np.float32)
+    row = np.repeat(np.arange(n), np.diff(csr.rowptr))
+    want = (2 * np.bincount(row, weights=(x * scale)[csr.colind], minlength=n) + 1).astype(np.float32)
+    dx, ds, dy = gbo.DeviceBuffer.from_numpy(x), gbo.DeviceBuffer.from_numpy(scale), gbo.DeviceBuffer(4 * n)
+    for _ in range(2):
+        g.bmv_float(dx, dy, 2.0, ds, 1.0)
+        assert np.array_equal(dy.to_numpy(np.float32, n), want)
