@@ -1150,16 +1150,17 @@ __device__ __forceinline__ double pr_row_update(long long i, double a, const flo
 }
 
 // Up to `iters` iterations of a PageRank-type loop in one cooperative launch
-// over the row lists (gather.cuh), one block an SM.  Warps take parts in turn, sum their rows and
-// update those that began in the part; the next part's columns load
-// meanwhile.  Rows that cross parts leave their shares in `head` / `tail` and
+// over the row lists (gather.cuh), one block an SM.  Warps take parts in turn,
+// sum their rows and update those that began in the part; the next part's
+// columns load meanwhile.  Rows that cross parts leave their shares in `head` / `tail` and
 // are finished after a grid barrier, a thread per part they end in; a second
 // barrier closes the iteration, after which every block reads the same error
 // and takes the same decision.  The iterate is read with plain loads: the
 // barriers' fences make the other blocks' writes visible to them.
 //
 // Bound by the gathers of the iterate (a 32-byte sector of L2 each where L1
-// misses) and the instructions around them.  Per iteration: R-MAT 21 (62 M
+// misses), the instructions around them (79 a set bit at R-MAT 20, issue 59 %)
+// and the half of the warps that 64 registers leave room for.  Per iteration: R-MAT 21 (62 M
 // set bits) 580 us as row-word walks in a loop graph, 226 now; R-MAT 18 140
 // and 38; 1,003 vertices 21 and 9 (two barriers); a mesh of 640,000 vertices
 // 32 and 28.  On the way, R-MAT 21: a block of 256 threads per part 316 (its
@@ -1376,9 +1377,9 @@ __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ 
 // forest in the caller's label array whose links always go from a higher to a
 // lower vertex, so a component's root is its smallest vertex.  Three edges per
 // vertex (its first, last and second neighbour) link most of a graph's largest
-// component; a sample of the labels
-// names it, and only the vertices outside it go through all their edges (an
-// edge between the two sides is seen from the outside one: P is symmetric).
+// component; a sample of the labels names it, and only the vertices outside it
+// go through all their edges (an edge between the two sides is seen from the
+// outside one: P is symmetric).
 //
 // Bound by the random accesses to the labels (a handful per vertex).  The
 // FastSV loop this replaces gathered a label per set bit in each of its four

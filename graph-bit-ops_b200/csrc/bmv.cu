@@ -513,19 +513,25 @@ __global__ void k_terms(const float* __restrict__ x, const float* __restrict__ s
     z[j] = x[j] * scale[j];
 }
 
-// Where the gathers of x and scale are what a product waits for -- wide tiles
-// (b = 64) and long block rows among short ones -- the terms are laid out first
-// and a set bit takes one gather instead of two: R-MAT 20, b = 32 492 -> 476 us,
-// b = 64 2,614 -> 2,520; R-MAT of 150,001 rows, b = 16 195 -> 184.  Else the
-// gathers hide behind the words, and the launch is lost: uniform of 60,001 rows,
-// 24 a row, b = 4 42.0 -> 45.9, b = 32 29.2 -> 33.4; of 1,048,576 rows, b = 32
-// 323 -> 324.  The same holds for few tiles.  The buffer comes from the pool,
-// which a stream under capture does not take.  (Degrees are not read ahead: a
-// row pointer need only reach as far as the set columns.)
+// Laying the terms out first saves a gather of `scale` per set bit for a launch
+// and a pass over the columns (4 us and 3 for a million of them).  That pays from
+// few tiles on where a product waits for its gathers -- 64 columns a word, or a
+// long block row among short ones -- and else only for many tiles, met 16 times a
+// column.  Without / with (us): b = 64, uniform of 60,001 rows, 24 a row (0.7 M
+// tiles) 211 / 203, of 30,001 rows, 8 a row (0.1 M) 48 / 50; R-MAT 20 b = 32 508 /
+// 473, of 60,001 rows (0.4 M) 127 / 119, of 30,001 rows b = 16 (0.3 M) 42 / 43;
+// uniform, 24 a row, b = 32, of 1,048,576 rows (25 M) 337 / 325, of 150,001 (3.3 M)
+// 59.7 / 59.7, of 60,001 28.9 / 32.3, 8 a row of 1,048,576 (8.4 M) 131 / 134, b = 4,
+// 24 a row of 400,003 (9.6 M) 138 / 133; mesh of 1,048,576 rows, b = 4 28.9 / 34.8.
+// The buffer comes from the pool, which a stream under capture does not take.
+// (Degrees are not read ahead: a row pointer need only reach as far as the set
+// columns.)
 float* float_terms(const gbo_graph* g, const GView& v, const float* x, const float* scale, cudaStream_t s) {
   const bool skewed = (long long)g->longest * g->nbr > 12 * g->nblk;
-  const long long least = g->b >= 16 && skewed ? 1ll << 20 : g->b == 64 ? 1ll << 21 : 1ll << 62;
-  if (!scale || v.ncols <= 0 || g->nblk < least) return nullptr;
+  const bool waits = g->b == 64 || (skewed && g->b >= 16);
+  const long long least = waits ? 1ll << 19 : skewed ? 1ll << 21 : 1ll << 23;
+  const long long met = waits || skewed ? 2 : 16;
+  if (!scale || v.ncols <= 0 || g->nblk < std::max(least, met * v.ncols)) return nullptr;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   float* z = nullptr;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||

@@ -1,5 +1,7 @@
-// Row lists of a ROW-layout graph and the balanced gather over them, for the
+// Row lists of a ROW-layout graph, and the balanced gather over them for the
 // iterations that gather one value per set bit (PageRank and its variants).
+// Connected components, triangle counts (tc.cu) and multi-source BFS with wide
+// frontier rows (ms_kernels.cuh) walk the same lists in their own ways.
 //
 // For a value gather the tiles only get in the way: R-MAT graphs hold 1.1 set
 // bits per non-empty row word, and walking words dealt a warp's lanes uneven

@@ -38,7 +38,8 @@ struct gbo_graph {
   unsigned* rowword = nullptr;  // b = 32 ROW: the non-empty row words, packed in tile order
   long long* item_wbase = nullptr;  // index in rowword of every work item's first word
   long long nrowword = 0;
-  // b = 32 ROW, built on first BFS use (build_rws): every row's non-empty
+  // b = 32 ROW, built on first use by a BFS or a multi-source BFS that walks
+  // them (build_rws): every row's non-empty
   // row words with their block columns in ascending block-column order; the
   // first kRwsHead entries of the 32 rows of a block row entry-major, the
   // rest in per-row tails
@@ -46,7 +47,7 @@ struct gbo_graph {
   uint2* rws_tail = nullptr;       // entries past the head, row after row
   long long* rws_tail_ptr = nullptr;  // nbr * 32 + 1 offsets into rws_tail
   // rows whose tails are longer than kRwsLongTail, cut into chunks of at most
-  // kRwsChunk tail entries, for kernels that must read whole rows (PageRank):
+  // kRwsChunk tail entries, for the multi-source BFS (a warp per chunk):
   // long row q owns chunks [rws_long_chunk0[q], rws_long_chunk0[q + 1])
   int rws_nlong = 0;
   long long rws_nchunk = 0;
@@ -58,7 +59,8 @@ struct gbo_graph {
   long long* rws_chunk_end = nullptr;
   unsigned* rws_longbits = nullptr;    // nbr words: bit 31 - r set when row 32R + r is long
   // the set columns of every row and the parts of a balanced walk over them
-  // (gather.cuh), built on first PageRank-type use
+  // (gather.cuh), built by the first PageRank-type loop, connected components,
+  // triangle count over lists or multi-source BFS with k > 64
   long long* gl_ptr = nullptr;  // nrows + 1
   int* gl_col = nullptr;
   void* gl_part = nullptr;      // gl_nparts parts (GatherPart)
@@ -125,7 +127,7 @@ int build_rowwords(gbo_graph* g, cudaStream_t stream);
 constexpr int kRwsHead = 8;
 constexpr unsigned kRwsNone = 0xffffffffu;
 // Tails longer than this are walked by a whole warp (BFS) or cut into
-// chunks of kRwsChunk entries spread over warps (PageRank).
+// chunks of kRwsChunk entries spread over warps (multi-source BFS).
 constexpr int kRwsLongTail = 64;
 constexpr int kRwsChunk = 512;
 // Row-word slices of a b = 32 ROW graph -> g->rws_* (no-op for other graphs

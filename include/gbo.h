@@ -162,8 +162,11 @@ GBO_API int gbo_graph_from_csr(const int* rowptr, const int* colind, int nrows,
 /* Wrap caller-owned device B2SR buffers (not copied, not freed).  d_outdeg
  * may be NULL (then PageRank entry points return GBO_ERR_INVALID).  The
  * work schedule and, for 32x32 ROW tiles, the per-tile occupancy words and
- * packed non-empty row words are derived from the buffers here, so their
- * contents must not change while the graph is in use. */
+ * packed non-empty row words are derived from the buffers here; the row lists
+ * (any width, ROW), the neighbour lists of triangle counts and the row-word
+ * slices (32x32 ROW) by the first later call that walks them (PageRank, PPR,
+ * components, triangle counts, BFS, multi-source BFS).  All are kept with the
+ * graph, so the buffers' contents must not change while it is in use. */
 GBO_API int gbo_graph_wrap_b2sr(int nrows, int ncols, int tile_bits, int layout,
                         int nblocks, const int* d_bsrRowPtr,
                         const int* d_bsrColInd, const void* d_bsrVal,

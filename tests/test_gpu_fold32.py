@@ -66,7 +66,8 @@ def test_terms_beforehand(gbo, orc, gpu, b):
 
 @pytest.mark.parametrize("b", [8, 16, 32, 64])
 def test_terms_beforehand_on_a_skewed_graph(gbo, gpu, b):
-    """A million tiles and a hub row far past the others (b = 8: not laid out)."""
+    """A million tiles, 3.5 a column, and a hub row far past the others (b = 8:
+    not laid out)."""
     rng = np.random.default_rng(b)
     n = 300_007
     src = np.concatenate([rng.integers(0, n, 1_150_000), np.full(n, 77)])
