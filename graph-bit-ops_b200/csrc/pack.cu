@@ -99,12 +99,16 @@ __device__ __forceinline__ void consume(RowCursor& c, const int* __restrict__ co
 // at most: fill_words, count_words) -- or to be a straggler, with more than
 // 1 / kStragglers of the graph's work and kAboveMean times a slab's mean, which
 // the merge would finish last: no more than kStragglers slabs are, so the pass
-// stays linear in the graph.  Where the sides meet (uniform graphs, merge /
-// wide, us): fill b = 4, 2.7 words a tile 75 / 108; b = 8, 2.7 148 / 148; b = 16,
-// 8 265 / 288; b = 32, 10.7 17,525 / 21,143; b = 64, 1.4 15,045 / 15,376; count
-// b = 8, 10.7 words an entry 276 / 201, 42.7 869 / 1,216; b = 16, 42.7 6,141 /
-// 5,020.  Stragglers (R-MAT 19 / 22, b = 8, fill, us): 16,384 and 4 times the
-// mean 741 / 12,857, 32,768 and 2 533 / 17,369, 65,536 and 2 539 / 20,756.
+// stays linear in the graph -- or to be one of so few slabs that the bitmaps of
+// all of them take less than its own merge (kFewSlabs: a block goes through a
+// word in 2.3 ns, the merge through a step in 240 and more; 3 rows of 3,000
+// entries, 30 M columns, b = 4 2,576 / 238 us, 100 rows of 700, 4 M columns, b = 8
+// 954 / 127).  Where the sides meet (uniform graphs, merge / wide, us): fill b = 4,
+// 2.7 words a tile 75 / 108; b = 8, 2.7 148 / 148; b = 16, 8 265 / 288; b = 32,
+// 10.7 17,525 / 21,143; b = 64, 1.4 15,045 / 15,376; count b = 8, 10.7 words an
+// entry 276 / 201, 42.7 869 / 1,216; b = 16, 42.7 6,141 / 5,020.  Stragglers (R-MAT
+// 19 / 22, b = 8, fill, us): 16,384 and 4 times the mean 741 / 12,857, 32,768 and 2
+// 533 / 17,369, 65,536 and 2 539 / 20,756.
 // Without this rule the fill of uniform graphs of 2^23 vertices, 24 a row, took
 // 2,574 ms at b = 4 and 736 at b = 8 (merge: 4.3, 4.9), the count of a mesh of
 // that size at b = 32 1,299 us (merge: 247).
@@ -124,6 +128,7 @@ __host__ __device__ constexpr int count_words() {
 }
 constexpr long long kStragglers = 32768;
 constexpr int kAboveMean = 2;
+constexpr long long kFewSlabs = 4096;
 constexpr int kUnitEntries = 2048;
 
 // Units of a slab with this many entries.
@@ -201,9 +206,9 @@ __global__ void __launch_bounds__(kPackTPB) k_pack(const int* __restrict__ rowpt
       const int tiles = slab_ok ? bsr_rowptr[slab + 1] - bsr_rowptr[slab] : 0;
       const long long steps = max(tiles, longest);
       w = slab_ok && (tiles > merge_tiles<B>() || longest > kMergeRow) &&
-          (steps * fill_words<B>() >= words || steps * stragglers >= bsr_rowptr[nbr]);
+          (steps * fill_words<B>() >= words || steps * stragglers >= bsr_rowptr[nbr] || steps * kFewSlabs >= words * nbr);
     } else {
-      const bool straggler = entries * stragglers >= nnz;
+      const bool straggler = entries * stragglers >= nnz || entries * kFewSlabs >= words * nbr;
       w = slab_ok && entries > kMergeEntries && (entries * count_words<B>() >= words || straggler);
       if (__any_sync(0xffffffffu, w)) {
         int first = c0.head, last = c0.pos < c0.end ? colind[c0.end - 1] : -1;
