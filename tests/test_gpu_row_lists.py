@@ -131,6 +131,8 @@ def test_stream_with_a_part_of_the_sms(gbo, gpu):
     drv = pytest.importorskip("cuda.bindings.driver")
 
     def ok(r):
+        if r[0] in (drv.CUresult.CUDA_ERROR_NOT_SUPPORTED, drv.CUresult.CUDA_ERROR_NOT_PERMITTED):
+            pytest.skip("no green contexts here")
         assert r[0] == drv.CUresult.CUDA_SUCCESS, r[0]
         return r[1] if len(r) == 2 else r[1:]
 
